@@ -626,12 +626,13 @@ DtArgs dt_args(axj_handle* h, int advance) {
   d.flags = h->flags;
   d.time = h->time;
   d.advance = advance;
+  d.nblk = h->dt_blocks;
   d.c = h->c;
   return d;
 }
 
 int enqueue_dt(axj_handle* h, int advance) {
-  AXJ_CUDA(h, launch_dt(dt_args(h, advance), h->dt_blocks, h->stream));
+  AXJ_CUDA(h, launch_dt(dt_args(h, advance), h->stream));
   return AXJ_OK;
 }
 
@@ -1336,6 +1337,7 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
   c.r_top = rvec[(Nr - 1) * Nz];
   c.inv_gam = 1.0 / prm->gam;
   c.inv_Re = 1.0 / prm->Re;
+  c.inv_RePr = 1.0 / (prm->Re * prm->Pr);
   c.gam_RePr = prm->gam / (prm->Re * prm->Pr);
   c.gg1_Re = prm->gam * (prm->gam - 1.0) / prm->Re;
   c.do_viscous = prm->do_viscous_terms == 1;
@@ -1465,8 +1467,8 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
   h->harm = dalloc<double>(h, 5, &rc);
   h->flags = dalloc<int>(h, 1, &rc);
 
-  h->counter = dalloc<unsigned int>(h, 1, &rc);
-  h->dt_blocks = dt_grid_blocks();
+  h->counter = dalloc<unsigned int>(h, 2, &rc);
+  h->dt_blocks = dt_grid_blocks((int)Nz, (int)Nr);
   h->partial = dalloc<double>(h, h->dt_blocks, &rc);
   h->tiles_int = dalloc<int2>(h, std::max<size_t>(tint.size(), 1), &rc);
   h->tiles_gen = dalloc<int2>(h, std::max<size_t>(tgen.size(), 1), &rc);
@@ -2683,8 +2685,9 @@ int batch_build_tables(axj_batch* b) {
     if (int rc = bupload(b, &b->zr_argv, zv)) return rc;
     if (int rc = bupload(b, &b->zr_items, items)) return rc;
   }
-  // dt: the same number of blocks for every instance (the handles' partial arrays hold 592)
-  b->dt_blocks = (int)std::min<long long>(592, std::max<long long>(1, b->max_pts / (DT_THREADS * 8)));
+  // dt: the grid covers the largest instance's blocks
+  b->dt_blocks = 1;
+  for (int k = 0; k < n; ++k) b->dt_blocks = std::max(b->dt_blocks, b->h[k]->dt_blocks);
   return batch_tiles(b, true);
 }
 

@@ -20,6 +20,7 @@ namespace axj {
 constexpr int TZ = 32;
 constexpr int TR = 16;
 constexpr int STAGE_THREADS = 256;
+constexpr int DT_THREADS = 256;  // ComputeTimeStep
 
 // Halo of the two tile classes. Interior tiles only use the interior SBP rows
 // (reach 2); general tiles (domain edges, patch strips, blanked points, face
@@ -82,8 +83,8 @@ struct Consts {
   double r_top;   // r(i, Nr): sponge normalisation (ModBC.f90:571)
   double harm_amp, harm_omega;  // harmonic forcing (control_forcing == 2): A, 2 pi St U_j
   // per-run factors of the right-hand side, formed once on the host: 1/gam, 1/Re,
-  // gam/(Re Pr), gam (gam - 1)/Re
-  double inv_gam, inv_Re, gam_RePr, gg1_Re;
+  // gam/(Re Pr), gam (gam - 1)/Re; 1/(Re Pr) of the time step
+  double inv_gam, inv_Re, gam_RePr, gg1_Re, inv_RePr;
   int do_viscous;
   int shock_capturing;
   int control_forcing;  // 0 off, 1 feedback (ControlForcingTerms), 2 harmonic source

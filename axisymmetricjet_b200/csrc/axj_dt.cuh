@@ -1,0 +1,161 @@
+// axj_dt.cuh -- the point scan of ComputeTimeStep (ModInputOutput.f90:389-438), shared by the
+// handle-based and the allocation-free time-step kernels.
+//
+// dt is the minimum of CFL / x over the points, x the point's inviscid plus viscous rate. In
+// FP64 x costs about fifty instructions per point (two square roots, T**0.666 with its table
+// loads), which bound the kernels at 36-52 us for 2.8 M points when the 24 B/point they read
+// take 10 us; but only the points near the largest x need it. A block therefore first forms an
+// FP32 estimate of x for its points with the approximate square root, log2 and exp2 units
+// (relative error of the parts well below 1e-5), takes the largest estimate, and evaluates
+// x in FP64 only where the estimate lies within DT_SCREEN of the parts' magnitudes of that.
+// The margin is an order of magnitude wider than the estimate's error, so the point of the
+// largest x is always among them and the result is the full FP64 scan's, bit for bit.
+// Estimates that are not finite (NaN or infinite inputs, FP32 overflow) are always evaluated
+// in FP64. The largest lower bound seen so far is handed from block to block through a word
+// in global memory (a hint: any value it holds is a valid bound), so that most blocks evaluate
+// no point in FP64 at all.
+// Measured at 4400 x 640 on a B200: the allocation-free kernel 51.4 -> 19.7 us (a call 57.4 ->
+// 22.6 us), the handle's 35.7 -> 23.0 us; what remains is issue (62 % of the active cycles) and
+// the launch's head and tail. Unscreened at 512 x 128 (one strip row per warp, a grid sized to
+// the points): 6.8 -> 5.5 us, where the screened form took 12.4.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "axj_common.cuh"
+
+namespace axj {
+
+// A warp takes a strip of 32 columns by DT_K rows (1 row where the scan is not screened): the
+// z metric is loaded and converted once per strip, the row's by one lane, and rows shorter
+// than a block waste at most part of a strip.
+constexpr int DT_K = 4;
+constexpr int DT_WARPS = DT_THREADS / 32;
+// Grids up to this many points are scanned in FP64 throughout, one point per thread: with
+// under two points for every resident thread the screen's extra barrier and second pass cost
+// more than the FP64 work they save.
+constexpr long long DT_FULL = 148ll * 8 * DT_THREADS;
+__host__ __device__ constexpr bool dt_screened(long long npts) { return npts > DT_FULL; }
+__host__ __device__ constexpr int dt_rows(bool screen) { return screen ? DT_K : 1; }
+// Strips of a grid, and the blocks that take one strip per warp.
+__host__ __device__ inline long long dt_strips(int Nz, int Nr, bool screen) {
+  const int K = dt_rows(screen);
+  return (long long)((Nz + 31) / 32) * ((Nr + K - 1) / K);
+}
+constexpr long long DT_WAVE = 148 * 4;  // blocks of a screened scan: one resident wave
+__host__ __device__ inline long long dt_blocks(int Nz, int Nr, bool screen) {
+  const long long b = (dt_strips(Nz, Nr, screen) + DT_WARPS - 1) / DT_WARPS;
+  return screen && b > DT_WAVE ? DT_WAVE : b;
+}
+constexpr float DT_SCREEN = 1.220703125e-4f;   // 2**-13
+constexpr float DT_TINY = 1.0e-30f;            // absolute margin (FP32 underflow, flushed subnormals)
+
+__device__ __forceinline__ float f_sqrt(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float f_lg2(float x) {
+  float y;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float f_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+struct DtScan {
+  const double* U;       // 5 planes of Nr rows, pitch P
+  long long P, plane;    // row pitch, plane size
+  int Nz, Nr;
+  const double* dxidz;
+  const double* detadr;
+  bool phys;     // sound speed from the point's T (else sqrt_stale)
+  float sqrt_stale, inv_Re, inv_RePr;
+};
+
+// One strip of 32 columns x K rows, by one warp; SCREEN: as above, else every point in FP64.
+// blanked(o): whether the point at offset o is blanked (counted in nblank); exact(i, j, o): the
+// FP64 evaluation. sL: the largest lower bound the block knows (float bits in shared memory,
+// zeroed by the caller before a barrier; it only grows, any value it holds is a valid bound, and
+// no warp waits for another's); hint: the launch's.
+template <int K, bool SCREEN, class Blanked, class Exact>
+__device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, unsigned* sL, unsigned* hint,
+                                              int& nblank, Blanked blanked, Exact exact) {
+  // (a grid that fits the device has far fewer than 2**31 strips)
+  const unsigned ncs = (unsigned)(s.Nz + 31) / 32u, lane = threadIdx.x & 31u;
+  const unsigned rg = strip / ncs;
+  const int j0 = (int)(rg * K), nrow = min(K, s.Nr - j0);
+  const int iu = (int)((strip - rg * ncs) * 32u + lane), i = min(iu, s.Nz - 1);
+  const long long o0 = (long long)j0 * s.P + i;
+  unsigned cand = 0;  // rows to evaluate in FP64
+  if constexpr (SCREEN) {
+    // every load of the strip first (none depends on another), then the estimates
+    double vr[K], vz[K], tt[K];
+    bool bl[K];
+    const double* u = s.U + o0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const long long o = min(k, nrow - 1) * s.P;  // rows past the grid repeat the last one
+      bl[k] = blanked(o0 + o);
+      vr[k] = __ldg(u + s.plane + o);
+      vz[k] = __ldg(u + 3 * s.plane + o);
+      tt[k] = __ldg(u + 4 * s.plane + o);
+    }
+    const float x = (float)__ldg(s.dxidz + i);
+    const float yl = (float)__ldg(s.detadr + j0 + min((int)lane, nrow - 1));
+    float up[K];      // upper bound of x
+    float lo = 0.0f;  // largest lower bound
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const float y = __shfl_sync(0xffffffffu, yl, k);
+      const float Vr = (float)vr[k], Vz = (float)vz[k], T = (float)tt[k];
+      const float a = Vz * x, b = Vr * y;
+      const float g2 = x * x + y * y;
+      const float snd = s.phys ? f_sqrt(T) * f_sqrt(g2) : s.sqrt_stale * f_sqrt(g2);
+      const float mu = f_ex2(0.666f * f_lg2(T));
+      const float lam = (0.6f - 2.0f / 3.0f) * mu;
+      const float mx = fmaxf(fmaxf(mu, lam) * s.inv_Re, mu * s.inv_RePr);
+      const float d = fabsf(x) + fabsf(y);
+      const float visc = 2.0f * mx * (d * d);
+      const float est = fabsf(a + b) + snd + visc;
+      const float mar = DT_SCREEN * (fabsf(a) + fabsf(b) + snd + fabsf(visc)) + DT_TINY;
+      up[k] = est + mar;
+      // (a repeated row or column counts once more: the same bound, no point of its own)
+      if (bl[k]) {
+        nblank = 1;
+      } else {
+        lo = fmaxf(lo, est - mar);  // (fmaxf drops a NaN)
+        if (k < nrow && iu < s.Nz) cand |= 1u << k;
+      }
+    }
+    // a lower bound that overflowed says nothing
+    const unsigned lob = lo <= 3.0e38f ? __float_as_uint(lo) : 0u;
+    const unsigned w = __reduce_max_sync(0xffffffffu, lob);
+    const unsigned b = max(*reinterpret_cast<volatile unsigned*>(sL), w);
+    if (lane == 0 && b == w) atomicMax(sL, w);
+    if (threadIdx.x == 0) {
+      const unsigned h = *reinterpret_cast<volatile unsigned*>(hint);
+      if (h > b) atomicMax(sL, h);  // for the strips to come
+      else if (h < b) atomicMax(hint, b);
+    }
+    const float thr = __uint_as_float(b);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (up[k] < thr) cand &= ~(1u << k);
+  } else {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (k < nrow && iu < s.Nz) {
+        if (blanked(o0 + k * s.P)) nblank = 1;
+        else cand |= 1u << k;
+      }
+  }
+#pragma unroll 1
+  for (int k = 0; k < K; ++k)
+    if ((cand >> k) & 1u) exact(i, j0 + k, o0 + k * s.P);
+}
+
+}  // namespace axj

@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "axj_dt.cuh"
 #include "axj_kernels.cuh"
 #include "axj_point.cuh"
 #include "axj_pow.cuh"
@@ -890,55 +891,61 @@ __device__ __forceinline__ double warp_min(double v) {
   return v;
 }
 
-// ComputeTimeStep over one instance with blocks blk = 0..nblk-1 (per-block minima in
-// a.partial, the last block to finish reduces them).
+// ComputeTimeStep over one instance with blocks blk = 0..a.nblk-1 (per-block minima in
+// a.partial, the last block to finish reduces them), each scanning strips of points
+// (axj_dt.cuh; SCREEN: FP32 estimates, FP64 only near the largest).
 // The minimum of dt = CFL / x over the points is CFL / (maximum of x): division by a
 // positive x is monotonic and correctly rounded, so the two agree exactly; the kernel
 // reduces x and divides once. Likewise max(mu/Re, lambda/Re) = max(mu, lambda)/Re. The
-// divisions by Re and Re Pr are products with the reciprocals (within an ulp of the
-// quotients). The stale T's square root is formed once. Blanked points contribute dt = 100
-// (ModInputOutput.f90:398-400). A thread's (i, j) advances by the grid stride without a
-// division per point.
-__device__ __forceinline__ void dt_body(const DtArgs& a, int blk, int nblk) {
-  const int Nz = a.g.Nz, Nr = a.g.Nr;
-  const long long n = (long long)Nz * Nr;
+// divisions by Re and Re Pr are products with the host's reciprocals (within an ulp of the
+// quotients). Blanked points contribute dt = 100
+// (ModInputOutput.f90:398-400).
+template <bool SCREEN>
+__device__ __forceinline__ void dt_body(const DtArgs& a, int blk) {
   const long long PL = a.g.plane;
   const bool phys = a.c.dt_mode == DT_PHYSICAL;
-  const double sqrtTst = sqrt(*a.staleT);
-  const double inv_Re = 1.0 / a.c.Re, inv_RePr = 1.0 / (a.c.Re * a.c.Pr);
-  double xm = 0.0;  // maximum of the denominators (0: no unblanked point yet)
+  const double Tst = *a.staleT;
+  double xm = 0.0;  // maximum of the denominators (0: no unblanked point evaluated yet)
   int bad = 0, blank = 0;
-  const long long stride = (long long)nblk * DT_THREADS;
-  const int sj = (int)(stride / Nz), si = (int)(stride - (long long)sj * Nz);
-  long long p = (long long)blk * DT_THREADS + threadIdx.x;
-  int j = (int)(p / Nz), i = (int)(p - (long long)j * Nz);
-  for (; p < n; p += stride, i += si, j += sj) {
-    if (i >= Nz) {  // i + si < 2 Nz: one carry at most
-      i -= Nz;
-      ++j;
-    }
-    const long long o = (long long)j * a.g.P + i;
-    if (desc_blank(__ldg(a.desc + o))) {
-      blank = 1;
-      continue;
-    }
-    const double Vr = __ldg(a.U + 1 * PL + o), Vz = __ldg(a.U + 3 * PL + o), T = __ldg(a.U + 4 * PL + o);
-    const double dxidz = __ldg(a.dxidz + i), detadr = __ldg(a.detadr + j);
-    const double mu = mu_k<double>(T);
-    const double beta = (3.0 / 5.0) * mu;
-    const double lambda = beta - (2.0 / 3.0) * mu;
-    // dt_point's denominator, term for term
-    const double inv = fabs(Vz * dxidz + Vr * detadr) + (phys ? sqrt(T) : sqrtTst) * sqrt(dxidz * dxidz + detadr * detadr);
-    double mx = (lambda > mu ? lambda : mu) * inv_Re;
-    const double k = mu * inv_RePr;
-    if (k > mx) mx = k;
-    const double sabs = fabs(dxidz) + fabs(detadr);
-    const double x = inv + 2.0 * mx * (sabs * sabs);
-    if (!isfinite(x)) bad = 1;  // NaN, or an infinite input (which would give dt = 0)
-    xm = fmax(xm, x);
-  }
   __shared__ double sred[DT_THREADS / 32];
   __shared__ bool last;
+  __shared__ unsigned sL;
+  if (threadIdx.x == 0) sL = 0u;
+  __syncthreads();
+  DtScan sc;
+  sc.U = a.U;
+  sc.P = a.g.P;
+  sc.plane = PL;
+  sc.Nz = a.g.Nz;
+  sc.Nr = a.g.Nr;
+  sc.dxidz = a.dxidz;
+  sc.detadr = a.detadr;
+  sc.phys = phys;
+  sc.sqrt_stale = f_sqrt((float)Tst);
+  sc.inv_Re = (float)a.c.inv_Re;
+  sc.inv_RePr = (float)a.c.inv_RePr;
+  unsigned* hint = a.counter + 1;
+  const unsigned nstrip = (unsigned)dt_strips(sc.Nz, sc.Nr, SCREEN);
+  for (unsigned st = blk * DT_WARPS + (threadIdx.x >> 5); st < nstrip; st += a.nblk * DT_WARPS)
+    dt_scan_strip<dt_rows(SCREEN), SCREEN>(
+        sc, st, &sL, hint, blank, [&](long long o) { return desc_blank(__ldg(a.desc + o)); },
+        [&](int i, int j, long long o) {
+          const double Vr = __ldg(a.U + 1 * PL + o), Vz = __ldg(a.U + 3 * PL + o), T = __ldg(a.U + 4 * PL + o);
+          const double dxidz = __ldg(a.dxidz + i), detadr = __ldg(a.detadr + j);
+          const double mu = mu_k<double>(T);
+          const double beta = (3.0 / 5.0) * mu;
+          const double lambda = beta - (2.0 / 3.0) * mu;
+          // dt_point's denominator, term for term
+          const double inv =
+              fabs(Vz * dxidz + Vr * detadr) + sqrt(phys ? T : Tst) * sqrt(dxidz * dxidz + detadr * detadr);
+          double mx = (lambda > mu ? lambda : mu) * a.c.inv_Re;
+          const double k = mu * a.c.inv_RePr;
+          if (k > mx) mx = k;
+          const double sabs = fabs(dxidz) + fabs(detadr);
+          const double x = inv + 2.0 * mx * (sabs * sabs);
+          if (!isfinite(x)) bad = 1;  // NaN, or an infinite input (which would give dt = 0)
+          xm = fmax(xm, x);
+        });
   const bool anyblank = __syncthreads_or(blank);
   xm = warp_max(xm);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -955,14 +962,14 @@ __device__ __forceinline__ void dt_body(const DtArgs& a, int blk, int nblk) {
       a.partial[blk] = v;
       __threadfence();
       const unsigned int done = atomicAdd(a.counter, 1u);
-      last = (done == (unsigned int)nblk - 1);
+      last = (done == (unsigned int)a.nblk - 1);
     }
   }
   __syncthreads();
   if (last) {
     __threadfence();
     double mm = 1.0e300;
-    for (int b = threadIdx.x; b < nblk; b += DT_THREADS) mm = fmin(mm, ((volatile double*)a.partial)[b]);
+    for (int b = threadIdx.x; b < a.nblk; b += DT_THREADS) mm = fmin(mm, ((volatile double*)a.partial)[b]);
     mm = warp_min(mm);
     if (lane == 0) sred[w] = mm;
     __syncthreads();
@@ -973,19 +980,25 @@ __device__ __forceinline__ void dt_body(const DtArgs& a, int blk, int nblk) {
       if (a.advance) *a.time = *a.time + r;
       if (r == 100.0) atomicOr(a.flags, 2);
       *a.counter = 0u;
+      *hint = 0u;  // the next state starts without a bound
     }
   }
 }
 
-__global__ void __launch_bounds__(DT_THREADS) dt_kernel(const DtArgs a) { dt_body(a, blockIdx.x, gridDim.x); }
+template <bool SCREEN>
+__global__ void __launch_bounds__(DT_THREADS, 4) dt_kernel(const DtArgs a) {
+  dt_body<SCREEN>(a, blockIdx.x);
+}
 
-// Batched: blockIdx.y = instance.
-__global__ void __launch_bounds__(DT_THREADS) dt_kernel_batch(const DtArgs* __restrict__ argv) {
+// Batched: blockIdx.y = instance; the grid covers the largest one's blocks.
+__global__ void __launch_bounds__(DT_THREADS, 4) dt_kernel_batch(const DtArgs* __restrict__ argv) {
   __shared__ __align__(16) DtArgs sa;
+  if ((int)blockIdx.x >= argv[blockIdx.y].nblk) return;
   for (int k = threadIdx.x; k < (int)(sizeof(DtArgs) / 8); k += blockDim.x)
     reinterpret_cast<unsigned long long*>(&sa)[k] = reinterpret_cast<const unsigned long long*>(argv + blockIdx.y)[k];
   __syncthreads();
-  dt_body(sa, blockIdx.x, gridDim.x);
+  if (dt_screened((long long)sa.g.Nz * sa.g.Nr)) dt_body<true>(sa, blockIdx.x);
+  else dt_body<false>(sa, blockIdx.x);
 }
 
 __global__ void harmonic_phase_kernel(const double* time, const double* dt, double omega, int rhs_mode, double* out) {
@@ -1008,17 +1021,13 @@ cudaError_t launch_harmonic_phase(const double* time, const double* dt, double o
 
 // Blocks of the dt kernel for the current device: as many as are resident at once (one
 // wave, every SM full), so that every thread's loads are in flight together.
-int dt_grid_blocks() {
-  int dev = 0, nsm = 148, per_sm = 4;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dt_kernel, DT_THREADS, 0) != cudaSuccess || per_sm < 1)
-    per_sm = 4;
-  return nsm * per_sm;
+int dt_grid_blocks(int Nz, int Nr) {
+  return (int)std::min<long long>(dt_blocks(Nz, Nr, dt_screened((long long)Nz * Nr)), DT_MAX_BLOCKS);
 }
 
-cudaError_t launch_dt(const DtArgs& a, int nblocks, cudaStream_t s) {
-  dt_kernel<<<nblocks, DT_THREADS, 0, s>>>(a);
+cudaError_t launch_dt(const DtArgs& a, cudaStream_t s) {
+  if (dt_screened((long long)a.g.Nz * a.g.Nr)) dt_kernel<true><<<a.nblk, DT_THREADS, 0, s>>>(a);
+  else dt_kernel<false><<<a.nblk, DT_THREADS, 0, s>>>(a);
   return cudaGetLastError();
 }
 

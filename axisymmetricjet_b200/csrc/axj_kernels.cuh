@@ -74,6 +74,7 @@ struct StageArgs {
   Consts c;
 };
 
+constexpr int DT_MAX_BLOCKS = 65536;  // per-block minima of ComputeTimeStep
 struct DtArgs {
   Grid g;
   const double* U;
@@ -82,11 +83,12 @@ struct DtArgs {
   const double* detadr;
   const double* staleT;
   double* partial;       // one per block
-  unsigned int* counter; // last-block-done counter, left at 0
+  unsigned int* counter; // last-block-done counter, then the scan's bound hint; both left at 0
   double* dt;            // result
   int* flags;            // bit 1: dt blow-up (every point blanked), bit 0: non-finite dt
   double* time;          // solution time, advanced by dt when advance != 0
   int advance;
+  int nblk;              // blocks of the instance (dt_grid_blocks)
   Consts c;
 };
 
@@ -149,8 +151,10 @@ void stage_boxes(bool gen, bool mixed, int* halo_w, int* halo_h, int* q_h, int* 
 // Boxes (elements, one plane deep) the sensor tile kernel expects for the stage input:
 // V_r / V_z box vw x vh, temperature box tw x th (rho uses the stage tile box).
 void sensor_boxes(bool gen, bool mixed, int* vw, int* vh, int* tw, int* th);
-cudaError_t launch_dt(const DtArgs& a, int nblocks, cudaStream_t s);
-int dt_grid_blocks();
+cudaError_t launch_dt(const DtArgs& a, cudaStream_t s);
+// Blocks of ComputeTimeStep over a grid (axj_dt.cuh): at most DT_MAX_BLOCKS; they loop over
+// its strips of points.
+int dt_grid_blocks(int Nz, int Nr);
 // cos(omega t_s) of the harmonic forcing: rhs_mode != 0: out[0] at t = *time; else
 // out[s], s = 1..4, at t_s = (*time - *dt) + c_s * *dt (the device time is t_n + dt).
 cudaError_t launch_harmonic_phase(const double* time, const double* dt, double omega, int rhs_mode, double* out,
@@ -202,8 +206,6 @@ cudaError_t launch_tgfilter(const Grid& g, const uint32_t* desc, const double* v
 // (9 = no filtering: blanked), pitch P; flags bit 2 is set if a bounded wait gives up.
 cudaError_t launch_tgfilter_z_inplace(const Grid& g, const uint32_t* desc, const unsigned char* zcode,
                                       const double* q, double* out, int nfield, int* flags, cudaStream_t s);
-
-constexpr int DT_THREADS = 256;
 
 // ---- batched launches: many solver instances per launch ----
 // Per-instance TMA maps of a batch, NM_BATCH per instance, at these indices:

@@ -16,21 +16,22 @@
 
 #include "../../include/axj.h"
 #include "axj_common.cuh"
+#include "axj_dt.cuh"
 #include "axj_kernels.cuh"
 #include "axj_point.cuh"
 #include "axj_pow.cuh"
 
 namespace {
 
-constexpr int NA_THREADS = 256;                       // one grid point per thread
-constexpr int NA_MAX_BLOCKS = 65536;                  // at most 16,777,216 points
+constexpr int NA_THREADS = axj::DT_THREADS;
+constexpr int NA_MAX_BLOCKS = 65536;                  // at most 16,777,216 points (256 each)
 constexpr long long NA_MAX_POINTS = (long long)NA_MAX_BLOCKS * NA_THREADS;
 constexpr int NA_COUNTER = NA_MAX_BLOCKS;             // slot of the completion counter
 constexpr int NA_BAD = NA_MAX_BLOCKS + 1;             // slot of the non-finite flag
 
-// The scratch: one partial minimum per block, then two 32-bit words (counter, flag)
-// kept in the slots after them. Every call shares it and it keeps the last call's
-// contents; each call clears the two words before its kernel runs.
+// The scratch: one partial minimum per block, then the 32-bit counter with the scan's bound
+// hint beside it, and the non-finite flag, in the slots after them. Every call shares it and
+// it keeps the last call's contents; each call clears those words before its kernel runs.
 static __device__ __align__(256) double g_dt_scratch[NA_MAX_BLOCKS + 2];
 // the tables of the FP64 power mu = T**0.666 (axj_pow.cuh), written by the first call on
 // each device
@@ -43,35 +44,51 @@ __device__ __forceinline__ double na_warp_min(double v) {
 }
 
 // Per-point dt of ComputeTimeStep (ModInputOutput.f90:395-416), block minimum, and the
-// last block to finish reduces the per-block minima.
-__global__ void __launch_bounds__(NA_THREADS)
+// last block to finish reduces the per-block minima. A block takes one strip per warp
+// of the shared point scan (axj_dt.cuh); the largest rate is the smallest dt only for a positive CFL, so
+// any other CFL turns the scan's screening off.
+template <bool SCREEN>
+__global__ void __launch_bounds__(NA_THREADS, 4)
     dt_noalloc_kernel(const double* __restrict__ U, long long P, long long plane, int Nz, int Nr,
                       const double* __restrict__ dxidz, const double* __restrict__ detadr,
                       const double* __restrict__ ibval, double staleT, axj::Consts c, double* scratch,
                       double* __restrict__ dt) {
   unsigned int* counter = reinterpret_cast<unsigned int*>(scratch + NA_COUNTER);
   unsigned int* bad = reinterpret_cast<unsigned int*>(scratch + NA_BAD);
-  const long long n = (long long)Nz * Nr;
-  const long long p = (long long)blockIdx.x * NA_THREADS + threadIdx.x;
+  const bool phys = c.dt_mode == axj::DT_PHYSICAL;
+  __shared__ unsigned sL;
+  if (threadIdx.x == 0) sL = 0u;
+  __syncthreads();
+  axj::DtScan sc;
+  sc.U = U;
+  sc.P = P;
+  sc.plane = plane;
+  sc.Nz = Nz;
+  sc.Nr = Nr;
+  sc.dxidz = dxidz;
+  sc.detadr = detadr;
+  sc.phys = phys;
+  sc.sqrt_stale = axj::f_sqrt((float)staleT);
+  sc.inv_Re = (float)c.inv_Re;
+  sc.inv_RePr = (float)c.inv_RePr;
   double v = 1.0e300;
-  if (p < n) {
-    const int j = (int)(p / Nz), i = (int)(p - (long long)j * Nz);
-    const long long o = (long long)j * P + i;
-    if (ibval && __ldg(ibval + o) == 0.0) {
-      v = 100.0;
-    } else {
-      const double Vr = __ldg(U + 1 * plane + o), Vz = __ldg(U + 3 * plane + o), T = __ldg(U + 4 * plane + o);
-      // mu = T**0.666 (AssignValues) from the table-driven power of the handle-based kernels
-      const double mu = axj::pow0666(T, g_na_pow);
-      const double beta = (3.0 / 5.0) * mu;
-      const double lambda = beta - (2.0 / 3.0) * mu;
-      const bool phys = c.dt_mode == axj::DT_PHYSICAL;
-      v = axj::dt_point(Vz, Vr, phys ? T : staleT, mu, lambda, mu, __ldg(dxidz + i), __ldg(detadr + j), c);
-      // an infinite input gives dt = 0, a finite-looking minimum: flag it with the NaNs
-      if (!isfinite(Vr) || !isfinite(Vz) || !isfinite(T)) atomicOr(bad, 1u);
-    }
-    if (!(v == v)) atomicOr(bad, 1u);
-  }
+  int blank = 0;
+  const unsigned nstrip = (unsigned)axj::dt_strips(Nz, Nr, SCREEN);
+  for (unsigned st = blockIdx.x * axj::DT_WARPS + (threadIdx.x >> 5); st < nstrip; st += gridDim.x * axj::DT_WARPS)
+    axj::dt_scan_strip<axj::dt_rows(SCREEN), SCREEN>(
+        sc, st, &sL, counter + 1, blank, [&](long long o) { return ibval && __ldg(ibval + o) == 0.0; },
+        [&](int i, int j, long long o) {
+          const double Vr = __ldg(U + 1 * plane + o), Vz = __ldg(U + 3 * plane + o), T = __ldg(U + 4 * plane + o);
+          // mu = T**0.666 (AssignValues) from the table-driven power of the handle-based kernels
+          const double mu = axj::pow0666(T, g_na_pow);
+          const double beta = (3.0 / 5.0) * mu;
+          const double lambda = beta - (2.0 / 3.0) * mu;
+          const double x = axj::dt_point(Vz, Vr, phys ? T : staleT, mu, lambda, mu, __ldg(dxidz + i), __ldg(detadr + j), c);
+          // an infinite input gives dt = 0, a finite-looking minimum: flag it with the NaNs
+          if (!isfinite(Vr) || !isfinite(Vz) || !isfinite(T) || !(x == x)) atomicOr(bad, 1u);
+          v = fmin(v, x);
+        });
+  if (blank) v = fmin(v, 100.0);
   __shared__ double sred[NA_THREADS / 32];
   __shared__ bool last;
   v = na_warp_min(v);
@@ -158,16 +175,21 @@ extern "C" int axj_compute_dt_noalloc(const double* d_pv, int64_t pitch, int64_t
   c.Re = params->Re;
   c.Pr = params->Pr;
   c.CFL = params->CFL;
+  c.inv_Re = 1.0 / c.Re;  // the screen's estimates; the points divide
+  c.inv_RePr = 1.0 / (c.Re * c.Pr);
   c.dt_mode = (int)params->dt_mode;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the counter and the flag must start at zero; the per-block minima are written
+  // the counter, the hint and the flag must start at zero; the per-block minima are written
   // before they are read
   cudaError_t e = cudaMemsetAsync(scratch + NA_COUNTER, 0, 2 * sizeof(double), s);
   if (e == cudaSuccess) {
     const long long n = Nz * Nr;
-    const int blocks = (int)((n + NA_THREADS - 1) / NA_THREADS);
-    dt_noalloc_kernel<<<blocks, NA_THREADS, 0, s>>>(d_pv, (long long)pitch, (long long)pitch * Nr, (int)Nz, (int)Nr,
-                                                    d_dxidz, d_detadr, d_ibval, stale_T, c, scratch, d_dt);
+    const bool screen = axj::dt_screened(n) && c.CFL > 0.0;
+    const long long need = axj::dt_blocks((int)Nz, (int)Nr, screen);
+    const int blocks = (int)(need < NA_MAX_BLOCKS ? need : NA_MAX_BLOCKS);
+    auto kernel = screen ? dt_noalloc_kernel<true> : dt_noalloc_kernel<false>;
+    kernel<<<blocks, NA_THREADS, 0, s>>>(d_pv, (long long)pitch, (long long)pitch * Nr, (int)Nz, (int)Nr, d_dxidz,
+                                         d_detadr, d_ibval, stale_T, c, scratch, d_dt);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
