@@ -1921,11 +1921,13 @@ int need_mlp_buffers(axj_handle* h) {
   return AXJ_OK;
 }
 
-// Forward and backward workspace of one batch (row-major, batch-major).
+// Workspace of the training kernels for batches of B points: partial gradients and losses,
+// the parameter-sized vectors, and (given or sampled batches that leave the device) X, T.
 struct TrainWs {
   int B = 0;
-  float *X = nullptr, *T = nullptr, *Z1 = nullptr, *H1 = nullptr, *Z2 = nullptr, *H2 = nullptr, *Y = nullptr,
-        *dY = nullptr, *dH2 = nullptr, *dH1 = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr, *loss = nullptr;
+  cudaStream_t stream = nullptr;
+  float *X = nullptr, *T = nullptr, *part = nullptr, *lpart = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr,
+        *loss = nullptr;
   int* step = nullptr;
   std::vector<void*> mem;
   ~TrainWs() {
@@ -1937,24 +1939,22 @@ struct TrainWs {
     if (*e == cudaSuccess) *e = cudaMalloc(&p, n * sizeof(T_) + 16);
     if (*e == cudaSuccess) {
       mem.push_back(p);
-      *e = cudaMemset(p, 0, n * sizeof(T_) + 16);
+      *e = cudaMemsetAsync(p, 0, n * sizeof(T_) + 16, stream);
     }
     return static_cast<T_*>(p);
   }
-  cudaError_t alloc(int B_, int nloss) {
+  // (zeroed in order on the stream that uses it)
+  cudaError_t alloc(cudaStream_t s, int B_, int nloss, bool xt) {
+    stream = s;
     B = B_;
     cudaError_t e = cudaSuccess;
-    const size_t b = (size_t)B;
-    X = get<float>(b * MLP_K1, &e);
-    T = get<float>(b * MLP_OUT, &e);
-    Z1 = get<float>(b * MLP_HID, &e);
-    H1 = get<float>(b * MLP_HID, &e);
-    Z2 = get<float>(b * MLP_HID, &e);
-    H2 = get<float>(b * MLP_HID, &e);
-    Y = get<float>(b * MLP_OUT, &e);
-    dY = get<float>(b * MLP_OUT, &e);
-    dH2 = get<float>(b * MLP_HID, &e);
-    dH1 = get<float>(b * MLP_HID, &e);
+    if (xt) {
+      X = get<float>((size_t)B * MLP_K1, &e);
+      T = get<float>((size_t)B * MLP_OUT, &e);
+    }
+    const size_t g = (size_t)train_grid(B);
+    part = get<float>(2 * g * MLP_NPARAM, &e);
+    lpart = get<float>(g, &e);
     grad = get<float>(MLP_NPARAM, &e);
     m = get<float>(MLP_NPARAM, &e);
     v = get<float>(MLP_NPARAM, &e);
@@ -1963,35 +1963,6 @@ struct TrainWs {
     return e;
   }
 };
-
-// Forward and backward pass over ws.X / ws.T; gradients (all parameters) into ws.grad,
-// the batch loss added to ws.loss[*ws.step].
-int forward_backward(axj_handle* h, TrainWs& w) {
-  const int B = w.B;
-  const float* P = h->mlp;
-  float* G = w.grad;
-  cudaStream_t s = h->stream;
-  const int ks = B >= 2048 ? B / 1024 : 1;
-  AXJ_CUDA(h, launch_gemm(false, true, B, MLP_HID, MLP_K1, w.X, MLP_K1, P + MLP_OFF_W1, MLP_K1, w.Z1, MLP_HID, 1, s));
-  AXJ_CUDA(h, launch_bias_gelu(w.Z1, P + MLP_OFF_B1, w.H1, B, MLP_HID, s));
-  AXJ_CUDA(h, launch_gemm(false, true, B, MLP_HID, MLP_HID, w.H1, MLP_HID, P + MLP_OFF_W2, MLP_HID, w.Z2, MLP_HID, 1, s));
-  AXJ_CUDA(h, launch_bias_gelu(w.Z2, P + MLP_OFF_B2, w.H2, B, MLP_HID, s));
-  AXJ_CUDA(h, launch_gemm(false, true, B, MLP_OUT, MLP_HID, w.H2, MLP_HID, P + MLP_OFF_W3, MLP_HID, w.Y, MLP_OUT, 1, s));
-  AXJ_CUDA(h, launch_bias(w.Y, P + MLP_OFF_B3, B, MLP_OUT, s));
-  AXJ_CUDA(h, launch_loss(w.Y, w.T, w.dY, w.loss, w.step, B, s));
-  AXJ_CUDA(h, cudaMemsetAsync(G, 0, sizeof(float) * MLP_NPARAM, s));
-  AXJ_CUDA(h, launch_gemm(true, false, MLP_OUT, MLP_HID, B, w.dY, MLP_OUT, w.H2, MLP_HID, G + MLP_OFF_W3, MLP_HID, ks, s));
-  AXJ_CUDA(h, launch_colsum(w.dY, G + MLP_OFF_B3, B, MLP_OUT, s));
-  AXJ_CUDA(h, launch_gemm(false, false, B, MLP_HID, MLP_OUT, w.dY, MLP_OUT, P + MLP_OFF_W3, MLP_HID, w.dH2, MLP_HID, 1, s));
-  AXJ_CUDA(h, launch_gelu_bwd(w.dH2, w.Z2, B * MLP_HID, s));
-  AXJ_CUDA(h, launch_gemm(true, false, MLP_HID, MLP_HID, B, w.dH2, MLP_HID, w.H1, MLP_HID, G + MLP_OFF_W2, MLP_HID, ks, s));
-  AXJ_CUDA(h, launch_colsum(w.dH2, G + MLP_OFF_B2, B, MLP_HID, s));
-  AXJ_CUDA(h, launch_gemm(false, false, B, MLP_HID, MLP_HID, w.dH2, MLP_HID, P + MLP_OFF_W2, MLP_HID, w.dH1, MLP_HID, 1, s));
-  AXJ_CUDA(h, launch_gelu_bwd(w.dH1, w.Z1, B * MLP_HID, s));
-  AXJ_CUDA(h, launch_gemm(true, false, MLP_HID, MLP_K1, B, w.dH1, MLP_HID, w.X, MLP_K1, G + MLP_OFF_W1, MLP_K1, ks, s));
-  AXJ_CUDA(h, launch_colsum(w.dH1, G + MLP_OFF_B1, B, MLP_HID, s));
-  return AXJ_OK;
-}
 
 Dataset dataset_of(axj_handle* h) {
   Dataset d;
@@ -2130,7 +2101,7 @@ int axj_dataset_sample(axj_handle* h, int64_t batch, int64_t seed, int64_t step,
   if (h->ds_n < 1) return fail(h, AXJ_ERR_ARG, "empty data set");
   AXJ_CUDA(h, cudaSetDevice(h->device));
   TrainWs w;
-  AXJ_CUDA(h, w.alloc((int)batch, 1));
+  AXJ_CUDA(h, w.alloc(h->stream, (int)batch, 1, true));
   const int st = (int)step;
   AXJ_CUDA(h, cudaMemcpyAsync(w.step, &st, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   AXJ_CUDA(h, launch_sample(dataset_of(h), h->norm, (unsigned long long)seed, w.step, (int)batch, w.X, w.T, h->stream));
@@ -2148,14 +2119,12 @@ int axj_mlp_grad(axj_handle* h, const float* X, const float* T, int64_t batch, a
   if (int rc = need_mlp_buffers(h)) return rc;
   AXJ_CUDA(h, cudaSetDevice(h->device));
   TrainWs w;
-  AXJ_CUDA(h, w.alloc((int)batch, 1));
-  std::vector<float> xb((size_t)batch * MLP_K1, 0.0f);
-  for (int64_t b = 0; b < batch; ++b)
-    for (int k = 0; k < MLP_IN; ++k) xb[b * MLP_K1 + k] = X[b * MLP_IN + k];
-  AXJ_CUDA(h, cudaMemcpyAsync(w.X, xb.data(), xb.size() * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+  AXJ_CUDA(h, w.alloc(h->stream, (int)batch, 1, true));
+  AXJ_CUDA(h, cudaMemcpyAsync(w.X, X, (size_t)batch * MLP_IN * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   AXJ_CUDA(h, cudaMemcpyAsync(w.T, T, (size_t)batch * MLP_OUT * sizeof(float), cudaMemcpyHostToDevice, h->stream));
-  int rc = forward_backward(h, w);
-  if (rc != AXJ_OK) return rc;
+  AXJ_CUDA(h, launch_train_pass(nullptr, h->norm, 0, 0, w.B, w.X, w.T, h->mlp, w.part, w.lpart, h->stream));
+  AXJ_CUDA(h, launch_train_update(w.part, w.lpart, w.B, nullptr, nullptr, nullptr, w.grad, w.loss, 0, 0.0f, 0.0f, 0.0f,
+                                  0.0f, h->stream));
   std::vector<float> g(MLP_NPARAM);
   float l = 0.0f;
   AXJ_CUDA(h, cudaMemcpyAsync(g.data(), w.grad, sizeof(float) * MLP_NPARAM, cudaMemcpyDeviceToHost, h->stream));
@@ -2198,15 +2167,13 @@ int axj_mlp_train(axj_handle* h, const axj_train_cfg* cfg, float* loss) {
     drop_graphs(h);
   }
   TrainWs w;
-  AXJ_CUDA(h, w.alloc((int)cfg->batch, (int)std::max<int64_t>(cfg->steps, 1)));
+  AXJ_CUDA(h, w.alloc(h->stream, (int)cfg->batch, (int)std::max<int64_t>(cfg->steps, 1), false));
   const Dataset d = dataset_of(h);
   for (int64_t it = 0; it < cfg->steps; ++it) {
-    AXJ_CUDA(h, launch_sample(d, h->norm, (unsigned long long)cfg->seed, w.step, w.B, w.X, w.T, h->stream));
-    int rc = forward_backward(h, w);
-    if (rc != AXJ_OK) return rc;
-    AXJ_CUDA(h, launch_adam(h->mlp, w.grad, w.m, w.v, MLP_NPARAM, w.step, (float)cfg->lr, (float)cfg->beta1,
-                            (float)cfg->beta2, (float)cfg->eps, h->stream));
-    AXJ_CUDA(h, launch_step_inc(w.step, h->stream));
+    AXJ_CUDA(h, launch_train_pass(&d, h->norm, (unsigned long long)cfg->seed, it, w.B, nullptr, nullptr, h->mlp, w.part,
+                                  w.lpart, h->stream));
+    AXJ_CUDA(h, launch_train_update(w.part, w.lpart, w.B, h->mlp, w.m, w.v, nullptr, w.loss, it, (float)cfg->lr,
+                                    (float)cfg->beta1, (float)cfg->beta2, (float)cfg->eps, h->stream));
   }
   if (loss && cfg->steps > 0)
     AXJ_CUDA(h, cudaMemcpyAsync(loss, w.loss, sizeof(float) * cfg->steps, cudaMemcpyDeviceToHost, h->stream));

@@ -101,25 +101,18 @@ struct Dataset {
 // of B points drawn from the data set by a counter-based hash of (seed, step, b).
 cudaError_t launch_sample(const Dataset& d, MlpNorm norm, unsigned long long seed, const int* step, int B, float* X,
                           float* T, cudaStream_t s);
-// C[M x N] (ldc) = opA(A) * opB(B), opA(m,k) = TA ? A[k*lda+m] : A[m*lda+k], opB(k,n) =
-// TB ? B[n*ldb+k] : B[k*ldb+n]. ksplit > 1 adds partial sums atomically (C zeroed first).
-cudaError_t launch_gemm(bool TA, bool TB, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
-                        float* C, int ldc, int ksplit, cudaStream_t s);
-// H = gelu(Z + b) in place of Z's copy: Z += b (kept for the backward pass), H = gelu(Z).
-cudaError_t launch_bias_gelu(float* Z, const float* b, float* H, int B, int N, cudaStream_t s);
-cudaError_t launch_bias(float* Z, const float* b, int B, int N, cudaStream_t s);
-// dY = 2 (Y - T) / B, loss[step] = sum (Y - T)^2 / B (accumulated atomically).
-cudaError_t launch_loss(const float* Y, const float* T, float* dY, float* loss, const int* step, int B,
-                        cudaStream_t s);
-// dZ = dH * gelu'(Z) (in place on dH).
-cudaError_t launch_gelu_bwd(float* dH, const float* Z, int n, cudaStream_t s);
-// db[n] += sum_b dZ[b][n]
-cudaError_t launch_colsum(const float* dZ, float* db, int B, int N, cudaStream_t s);
-// Adam on the flat parameter vector; step counter read from *step (0-based) and then
-// advanced by launch_step_inc.
-cudaError_t launch_adam(float* p, const float* g, float* m, float* v, int n, const int* step, float lr, float b1,
-                        float b2, float eps, cudaStream_t s);
-cudaError_t launch_step_inc(int* step, cudaStream_t s);
+// Forward and backward pass of one batch: drawn from the data set d as launch_sample draws
+// step `step`, or (d null) given as X [B x MLP_IN], T [B x MLP_OUT]. Partial parameter
+// gradients into part (2 train_grid(B) rows of MLP_NPARAM), partial losses into lpart
+// (train_grid(B)).
+int train_grid(int B);
+cudaError_t launch_train_pass(const Dataset* d, const MlpNorm& norm, unsigned long long seed, long long step, int B,
+                              const float* X, const float* T, const float* P, float* part, float* lpart,
+                              cudaStream_t s);
+// The sums of the partial gradients into g, or (g null) Adam's update of p, m, v with them as
+// step `step` (0-based); the batch loss into loss[step].
+cudaError_t launch_train_update(const float* part, const float* lpart, int B, float* p, float* m, float* v, float* g,
+                                float* loss, long long step, float lr, float b1, float b2, float eps, cudaStream_t s);
 // Per-channel sums / sums of squares of the data set's features and targets
 // (acc: 4 x (sum, sumsq) features, 2 x sumsq targets, count), for the normalisation.
 cudaError_t launch_dataset_stats(const Dataset& d, double* acc, cudaStream_t s);
