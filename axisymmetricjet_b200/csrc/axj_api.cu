@@ -119,6 +119,9 @@ struct axj_handle {
   // fused z/r filter: Q blocks, z and r code blocks, temperature blocks of the stage
   // buffers; the coefficient planes it writes, as boxes of the two tile classes
   CUtensorMap map_zrQ, map_zrZc, map_zrRc, map_zrT[5];
+  std::vector<int2> zr_rb;      // its row blocks (zr_row_blocks) and segment length
+  int2* zr_rblocks = nullptr;
+  int zr_seg = ZRK_BZ;
   CUtensorMap map_coef[2];
   // interior tiles as two CTAs of TR / 2 rows (int_rows == TR / 2, or a batch tuned so):
   // their boxes
@@ -402,9 +405,9 @@ int build_zr_maps(axj_handle* h) {
   const int nb = h->mixed ? NBUF : BUAF;
   int rc = make_map_zrq(h, &h->map_zrQ, h->Q);
   if (rc == AXJ_OK) rc = make_map_u8(h, &h->map_zrZc, h->zcode, ZRK_BZ, ZRK_NR);
-  if (rc == AXJ_OK) rc = make_map_u8(h, &h->map_zrRc, h->rcode, ZRK_BZ, ZRK_RB);
+  if (rc == AXJ_OK) rc = make_map_u8(h, &h->map_zrRc, h->rcode, ZRK_BZ, ZRK_RBC);
   for (int b = 0; b < nb && rc == AXJ_OK; ++b)
-    rc = make_map(h, &h->map_zrT[b], buf_ptr(h, b), 5, ZRK_BZ, ZRK_RB, 1, buf_f32(b));
+    rc = make_map(h, &h->map_zrT[b], buf_ptr(h, b), 5, ZRK_BZ, ZRK_RBC, 1, buf_f32(b));
   for (int cls = 0; cls < 2 && rc == AXJ_OK; ++cls) {
     int hw, hh, qh, tw, th, qlh;
     stage_boxes(cls == 1, h->mixed, &hw, &hh, &qh, &tw, &th, &qlh);
@@ -496,6 +499,65 @@ int launch_stage_kernels(axj_handle* h, int bin, int bout, int stage, int cm) {
   return AXJ_OK;
 }
 
+// Row blocks (first row, kind) of the fused z/r filter: compact ones wherever the r
+// filter's windows of their 40 rows stay within their ZRK_NR rows, wide ones of 30 elsewhere
+// (near walls inside the domain). rcode: r row codes, pitch P (9 = blanked: no window).
+std::vector<int2> zr_row_blocks(const std::vector<unsigned char>& rcode, int Nz, int Nr, int64_t P) {
+  std::vector<int> lo(Nr), hi(Nr), closed(Nr);  // rows the windows of a row reach; not all centred
+  for (int j = 0; j < Nr; ++j) {
+    const unsigned char* c = rcode.data() + (size_t)j * P;
+    int a = j, b = j;
+    for (int i = 0; i < Nz; ++i) {
+      if (i > 0 && c[i] == c[i - 1]) continue;
+      const int w = c[i];
+      if (w != 4) closed[j] = 1;
+      if (w >= 9) continue;
+      a = std::min(a, j + tg_w0(w));
+      b = std::max(b, j + tg_w0(w) + tg_len(w) - 1);
+    }
+    lo[j] = a;
+    hi[j] = b;
+  }
+  std::vector<int2> out;
+  for (int j = 0; j < Nr;) {
+    bool ok = true;
+    for (int r = j; r < std::min(Nr, j + ZRK_RBC) && ok; ++r)
+      ok = lo[r] >= j - ZRK_HRC && hi[r] < j - ZRK_HRC + ZRK_NR;
+    const int nr = ok ? ZRK_RBC : ZRK_RBW;
+    int cl = 0;
+    for (int r = j; r < std::min(Nr, j + nr); ++r) cl |= closed[r];
+    out.push_back(make_int2(j, (ok ? 1 : 0) | (cl ? 2 : 0)));
+    j += nr;
+  }
+  return out;
+}
+
+// Segment length (z positions) of the fused z/r filter over work items of Nz positions x
+// row blocks. A CTA's time goes with its blocks of 16 positions plus 2.5 (its warm-up blocks
+// run the recurrence alone); two CTAs of an SM take 1.03, three 1.2 times one's time, and more
+// than three run in turns. So small grids take the shortest segments that fill the SMs once and
+// large ones the longest that still leave three CTAs for each SM. Measured on a B200 (16 / 32 / 48
+// positions): 787 x 203 15.4 / 18.2 / 21.0 us; 1801 x 333 29.9 / 27.2 / 21.0, 64: 21.2;
+// 4400 x 640 176: 56.6, 96: 64, 272: 73.
+int zr_pick_segment(const std::vector<std::pair<int, int>>& work, int nsm) {
+  int kmax = 1;
+  for (const auto& w : work) kmax = std::max(kmax, (w.first + ZRK_BZ - 1) / ZRK_BZ);
+  int best = 1;
+  double tb = 1e300;
+  for (int k = 1; k <= kmax; ++k) {
+    long long n = 0;
+    for (const auto& w : work) n += (long long)((w.first + ZRK_BZ * k - 1) / (ZRK_BZ * k)) * w.second;
+    const long long c = (n + nsm - 1) / nsm;  // CTAs of the fullest SM
+    const double rest[3] = {0.0, 1.0, 1.03};
+    const double t = (k + 2.5) * (1.2 * (double)(c / 3) + rest[c % 3]);
+    if (t < tb) {
+      tb = t;
+      best = k;
+    }
+  }
+  return best * ZRK_BZ;
+}
+
 // The sensor chain of a stage input: the sensor tiles (quantities Q), then the fused
 // z filter / r filter / coefficient kernel, which leaves mu_eff, beta, kappa_eff in coef.
 ZrArgs zr_args(axj_handle* h, int seg) {
@@ -505,6 +567,8 @@ ZrArgs zr_args(axj_handle* h, int seg) {
   z.ramp = h->ramp;
   z.coef = h->coef;
   z.flags = h->flags;
+  z.rblocks = h->zr_rblocks;
+  z.nrblocks = (int)h->zr_rb.size();
   z.seg = seg;
   z.c = h->c;
   return z;
@@ -513,11 +577,7 @@ ZrArgs zr_args(axj_handle* h, int seg) {
 int enqueue_sensor_chain(axj_handle* h, int bin) {
   SensorArgs s = sensor_args(h, bin);
   AXJ_CUDA(h, launch_sensor_tiles_only(s, h->side, h->stream));
-  // about three CTAs per SM: segments of a multiple of ZRK_BZ positions, at least 64
-  const int nrb = (h->Nr + ZRK_RB - 1) / ZRK_RB;
-  const int nseg = std::max(1, (3 * 148) / nrb);
-  const int seg = (int)((h->Nz + nseg - 1) / nseg);
-  ZrArgs z = zr_args(h, std::max(64, (seg + ZRK_BZ - 1) / ZRK_BZ * ZRK_BZ));
+  const ZrArgs z = zr_args(h, h->zr_seg);
   ZrMaps m{&h->map_zrQ, &h->map_zrZc, &h->map_zrRc, &h->map_zrT[bin]};
   AXJ_CUDA(h, launch_zr(z, m, h->mixed, buf_f32(bin), h->stream));
   return AXJ_OK;
@@ -1293,6 +1353,7 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
     return fail(nullptr, AXJ_ERR_NODEVICE, "no CUDA device available");
+  int nsm = 148;
   if (prm->device < 0 || prm->device >= ndev)
     return fail(nullptr, AXJ_ERR_ARG, "device %lld not in 0..%d", (long long)prm->device, ndev - 1);
   {
@@ -1301,6 +1362,7 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
       return fail(nullptr, AXJ_ERR_NODEVICE, "device %lld is not an sm_100 (B200) GPU", (long long)prm->device);
     if (cudaSetDevice((int)prm->device) != cudaSuccess)
       return fail(nullptr, AXJ_ERR_NODEVICE, "cudaSetDevice(%lld) failed", (long long)prm->device);
+    nsm = prop.multiProcessorCount;
   }
   // tensor-product grid: z depends on i only, r on j only (the reference only
   // carries dxi/dz and deta/dr, ModDeriv.f90:57,108)
@@ -1446,6 +1508,9 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
     h->Qz = dalloc<double>(h, 3 * pl, &rc);
     h->coef = dalloc<double>(h, 3 * pl, &rc);
     h->rcode = dalloc<unsigned char>(h, pl, &rc);
+    h->zr_rb = zr_row_blocks(rcode, (int)Nz, (int)Nr, h->P);
+    h->zr_seg = zr_pick_segment({{(int)Nz, (int)h->zr_rb.size()}}, nsm);
+    h->zr_rblocks = dalloc<int2>(h, h->zr_rb.size(), &rc);
   }
   h->desc = dalloc<uint32_t>(h, pl, &rc);
   h->zcode = dalloc<unsigned char>(h, pl, &rc);
@@ -1488,6 +1553,7 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
   up(h->desc, desc.data(), desc.size() * sizeof(uint32_t));
   up(h->zcode, zcode.data(), zcode.size());
   if (h->rcode) up(h->rcode, rcode.data(), rcode.size());
+  if (h->zr_rblocks) up(h->zr_rblocks, h->zr_rb.data(), h->zr_rb.size() * sizeof(int2));
   up(h->faces, faces.data(), faces.size() * sizeof(int));
   up(h->dxidz, dxidz.data(), Nz * sizeof(double));
   up(h->ddxidxidz, ddxidxidz.data(), Nz * sizeof(double));
@@ -2633,20 +2699,18 @@ int batch_build_tables(axj_batch* b) {
     b->zthreads = bs;
     b->zsmem = sm;
     if (int rc = bupload(b, &b->zrows, rows)) return rc;
-    // the fused z/r filter over all instances: one segment length for the batch, about
-    // three CTAs per SM in all (segments of a multiple of ZRK_BZ, at least 64 positions)
-    long long work = 0;
-    for (int k = 0; k < n; ++k) work += (long long)b->h[k]->Nz * ((b->h[k]->Nr + ZRK_RB - 1) / ZRK_RB);
-    long long seg = std::max<long long>(64, (work + 3 * b->nsm - 1) / (3 * b->nsm));
-    seg = (seg + ZRK_BZ - 1) / ZRK_BZ * ZRK_BZ;
+    // the fused z/r filter over all instances: one segment length for the batch
+    std::vector<std::pair<int, int>> work;
+    for (int k = 0; k < n; ++k) work.push_back({b->h[k]->Nz, (int)b->h[k]->zr_rb.size()});
+    const int seg = zr_pick_segment(work, b->nsm);
     std::vector<ZrArgs> zv(n);
     std::vector<int4> items;
     for (int k = 0; k < n; ++k) {
       axj_handle* h = b->h[k];
-      zv[k] = zr_args(h, (int)seg);
-      const int nx = (int)((h->Nz + seg - 1) / seg), ny = (h->Nr + ZRK_RB - 1) / ZRK_RB;
-      for (int y = 0; y < ny; ++y)
-        for (int x = 0; x < nx; ++x) items.push_back(make_int4(x, y, k, 0));
+      zv[k] = zr_args(h, seg);
+      const int nx = (h->Nz + seg - 1) / seg;
+      for (const int2& rb : h->zr_rb)
+        for (int x = 0; x < nx; ++x) items.push_back(make_int4(x, rb.x, k, rb.y));
     }
     b->nzr_items = (int)items.size();
     if (int rc = bupload(b, &b->zr_argv, zv)) return rc;

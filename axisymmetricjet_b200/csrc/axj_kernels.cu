@@ -36,7 +36,7 @@ __constant__ double cC9[9];
 __constant__ float cC9f[9];
 // tables of the FP64 power mu = T**0.666 (axj_pow.cuh); read through the L1 cache, since
 // the points of a warp index them by their own T
-__device__ double gPowTab[POW_TAB];
+__device__ __align__(16) double gPowTab[POW_TAB];
 
 // mu = T**0.666 of the stage input: the table-driven FP64 power, or (FP32 stencils)
 // exp2f / log2f
@@ -44,6 +44,37 @@ template <typename R>
 __device__ __forceinline__ R mu_k(R T) {
   if constexpr (std::is_same<R, double>::value) return pow0666(T, gPowTab);
   else return mu_of_T<float>(T);
+}
+
+// mu of N stage inputs; in FP64 without a branch between them (their table loads and chains
+// interleave), the rare T outside the tables' range afterwards.
+template <int N, typename R>
+__device__ __forceinline__ void mu_n(const R (&T)[N], double (&mu)[N]) {
+  if constexpr (std::is_same<R, double>::value) {
+    bool ok = true;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      mu[u] = pow0666_table(T[u], gPowTab);
+      ok = ok && pow0666_in_range(T[u]);
+    }
+    if (!ok) {
+#pragma unroll 1
+      for (int u = 0; u < N; ++u) {
+        // (a dynamic index would put the arrays into local memory)
+        double t = T[0];
+#pragma unroll
+        for (int q = 1; q < N; ++q)
+          if (u == q) t = T[q];
+        const double v = pow0666(t, gPowTab);
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+          if (u == q) mu[q] = v;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < N; ++u) mu[u] = double(mu_of_T<float>(T[u]));
+  }
 }
 
 void upload_tables(const double sbp1[9][6], const double sbp2[9][6], const double tg[9][11],
@@ -2000,23 +2031,32 @@ __global__ void tgfilter_z_rows_kernel_batch(const SensorArgs* __restrict__ argv
 // :248-251; ModAssign.f90:20-23): from the unfiltered sensor quantities Q to
 // mu_eff = mu + mu*, beta = 0.6 mu + beta* and kappa_eff = mu + kappa* at every point.
 //
-// A CTA owns a segment of z positions (a multiple of ZRK_BZ) and ZRK_RB rows. It runs the
-// in-place z recurrence of PerformTGfilter(q, 1, q) for the three quantities on its rows
-// and ZRK_HR rows either side (the reach of the 11-point TG boundary rows of the r
-// filter): one thread per (quantity, row), marching along z in blocks of ZRK_BZ
-// positions. Segments start ZRK_WARM positions early from a zero history (the
+// A CTA owns a segment of z positions (a multiple of ZRK_BZ) and a row block (40 rows where the
+// r filter's windows stay near, else 30: ZRK_RBC, ZRK_RBW). It runs the in-place z recurrence of
+// PerformTGfilter(q, 1, q) for the three quantities on ZRK_NR rows, its own and those either
+// side that the r filter reads: one thread per (quantity, row), marching along z in blocks of
+// ZRK_BZ positions. Segments start ZRK_WARM positions early from a zero history (the
 // recurrence forgets its start: the dominant root of its feedback part is about 0.47, so
-// 0.47**64 < 1e-20); the first segment starts exactly at i = 0 from the reference's zero
+// 0.47**48 < 2e-16); the first segment starts exactly at i = 0 from the reference's zero
 // halo. The z-filtered block goes to shared memory, where the r filter
 // PerformTGfilter(q, 2, star) of the CTA's rows is applied with the point's r row, then
-// the C*Re(*Pr) scaling, the z ramp and mu = T**0.666 of the stage input.
+// the C*Re(*Pr) scaling, the z ramp and mu = T**0.666 of the stage input. A thread takes the
+// points of one position on 4 (3) consecutive rows, so that the centred filter's windows share
+// their loads: 3 x 12 values for four points where single points read 3 x 36. The points on
+// closure rows (and blanked ones) follow one per thread: within the threads' blocks of rows,
+// where a few threads take them one after the other, the CTAs along r = 0 and r = r_max
+// took two to five times the others' time and set the kernel's.
 // Blocks of Q arrive by TMA (128-byte swizzle: a thread reads its row's 16 values as 8
 // conflict-free 16-byte loads) into two slots: block k supplies the up to 10 values
 // right of block k-1 that the filter rows reach, and once both are in registers the
 // slot of block k-1 takes block k+1, which lands while block k-1 is filtered.
+// Measured on a B200 (FP64; before: 30 rows per CTA, a point per thread and round, the power's
+// branch between a thread's points, segments of at least 64 positions with 64 of warm-up):
+// 4400 x 640 64 -> 57 us, 1801 x 333 25.4 -> 21.2, 787 x 203 with a blanked lip 38 -> 15.4,
+// 96 x 64 15.2 -> 10. The FP64 pipe is the bound (336 instructions per thread and own block); it
+// is busy about half the time between the phases' barriers.
 // ---------------------------------------------------------------------------
-constexpr int ZRK_LANES = 3 * ZRK_NR;  // 156 recurrences per CTA
-constexpr int ZRK_WARM = 64;           // warm-up positions (4 blocks)
+constexpr int ZRK_LANES = 3 * ZRK_NR;  // 150 recurrences per CTA
 constexpr int ZRK_QROW = ZRK_BZ * 8;   // bytes of one row of a Q block (128)
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -2030,43 +2070,140 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 // (chunk index XOR row mod 8), as TMA writes it.
 __device__ __forceinline__ int zrk_chunk(int R, int c) { return R * ZRK_QROW + ((c ^ (R & 7)) << 4); }
 // The z-filtered block is stored transposed, [quantity][position][row] with ZRK_ZP rows
-// (odd: the r filter's reads, 16 positions x 2 rows per warp, and the recurrence's writes,
-// consecutive rows per warp, are free of bank conflicts), so the r filter's taps are
+// (odd: the r filter's reads, 16 positions at one row per half warp, and the recurrence's
+// writes, consecutive rows per warp, are free of bank conflicts), so the r filter's taps are
 // consecutive doubles at fixed offsets.
 constexpr int ZRK_ZP = ZRK_NR + 1;
+
+// One centred step of the z recurrence: the feed-forward sum of the point's value x0 and the
+// four right of it, then the filtered values left of it, h1 the newest, last, so that a step
+// waits one FMA for each of them (the reference sums left to right; the orders differ by
+// rounding only).
+__device__ __forceinline__ double zr_ff(double x0, double x1, double x2, double x3, double x4) {
+  double s = cTG[4][4] * x0;
+  s = s + cTG[4][5] * x1;
+  s = s + cTG[4][6] * x2;
+  s = s + cTG[4][7] * x3;
+  return s + cTG[4][8] * x4;
+}
+__device__ __forceinline__ double zr_fb(double s, double h4, double h3, double h2, double h1) {
+  s = s + cTG[4][0] * h4;
+  s = s + cTG[4][1] * h3;
+  s = s + cTG[4][2] * h2;
+  return s + cTG[4][3] * h1;
+}
 
 template <typename SIN>
 struct ZrSmem {
   static constexpr size_t qbytes = (size_t)ZRK_LANES * ZRK_QROW;
   static constexpr size_t qslot = (qbytes + 1023) / 1024 * 1024;
   static constexpr size_t zslot = ((size_t)3 * ZRK_BZ * ZRK_ZP * sizeof(double) + 1023) / 1024 * 1024;
+  static constexpr size_t rcslot = 640;
   static constexpr size_t oQ = 0;                                            // [2] Q blocks (swizzled)
   static constexpr size_t oZ = 2 * qslot;                                    // z-filtered block [3][16][ZRK_ZP]
   static constexpr size_t oZc = oZ + zslot;                                  // [2][ZRK_NR][16] z row codes
   static constexpr size_t zcbytes = (size_t)ZRK_NR * ZRK_BZ;
-  static constexpr size_t oT = oZc + 2 * 1024;                               // [2][ZRK_RB][16] T
-  static constexpr size_t tbytes = (size_t)ZRK_RB * ZRK_BZ * sizeof(SIN);
-  static constexpr size_t oRc = oT + 2 * ((tbytes + 127) / 128 * 128);       // [2][ZRK_RB][16] r row codes
-  static constexpr size_t rcbytes = (size_t)ZRK_RB * ZRK_BZ;
-  static constexpr size_t oW = oRc + 2 * 512;                                // [10][21] padded TG rows
+  static constexpr size_t oT = oZc + 2 * 1024;                               // [2][ZRK_RBC][16] T
+  static constexpr size_t tbytes = (size_t)ZRK_RBC * ZRK_BZ * sizeof(SIN);
+  static constexpr size_t oRc = oT + 2 * ((tbytes + 127) / 128 * 128);       // [2][ZRK_RBC][16] r row codes
+  static constexpr size_t rcbytes = (size_t)ZRK_RBC * ZRK_BZ;
+  static constexpr size_t oW = oRc + 2 * rcslot;                                // [10][21] padded TG rows
   static constexpr size_t bytes = oW + 10 * 21 * sizeof(double) + 1024;      // + alignment slack
   static constexpr uint32_t tx = (uint32_t)(qbytes + zcbytes + tbytes + rcbytes);
-  static_assert(zcbytes <= 1024 && rcbytes <= 512, "code slots");
+  static_assert(zcbytes <= 1024 && rcbytes <= rcslot && tbytes % 128 == 0, "code and T slots");
 };
 
-// The fused z/r filter for the CTA (bx, by): z positions bx * a.seg .., rows by * ZRK_RB ..
+__device__ __forceinline__ void zr_store(const ZrArgs& a, double* out, double ramp, double mu, double f0, double f1,
+                                         double f2) {
+  const long long PL = a.g.plane;
+  out[0] = mu + a.c.C_mu_Re * f0 * ramp;
+  out[PL] = (3.0 / 5.0) * mu + a.c.C_beta_Re * f1 * ramp;
+  out[2 * PL] = mu + a.c.C_kappa_Re_Pr * f2 * ramp;
+}
+
+// The r filter, scaling and coefficients of one thread's centred points: position p (z index i)
+// of a block on the NROW rows j0 + row0 .. (rows of the CTA), from the z-filtered block zb
+// whose first row is j0 - hr. tb, rcb: T and r codes of the CTA's rows.
+template <int NROW, typename SIN, typename R>
+__device__ __forceinline__ void zr_points(const ZrArgs& a, const double* zb, const SIN* tb, const unsigned char* rcb,
+                                          int p, int row0, int i, int j0, int hr) {
+  const long long P = a.g.P;
+  const int nrow = min(NROW, a.g.Nr - (j0 + row0));
+  if (nrow <= 0) return;
+  double mu[NROW], fv[3][NROW];
+  unsigned on = 0;
+  {
+    R T[NROW];
+#pragma unroll
+    for (int u = 0; u < NROW; ++u) {
+      T[u] = u < nrow ? R(tb[(row0 + u) * ZRK_BZ + p]) : R(1.0);
+      if (u < nrow && rcb[(row0 + u) * ZRK_BZ + p] == 4) on |= 1u << u;
+    }
+    mu_n<NROW, R>(T, mu);
+  }
+  // column of the first point in the transposed block: row j0 + row is Z row row + hr
+  const double* zc = zb + p * ZRK_ZP + row0 + hr;
+#pragma unroll
+  for (int f = 0; f < 3; ++f) {
+    const double* col = zc + f * ZRK_BZ * ZRK_ZP - 4;
+    double w[NROW + 8];
+#pragma unroll
+    for (int mm = 0; mm < NROW + 8; ++mm) w[mm] = col[mm];
+#pragma unroll
+    for (int u = 0; u < NROW; ++u) {
+      double s = cTG[4][0] * w[u];
+#pragma unroll
+      for (int mm = 1; mm < 9; ++mm) s = s + cTG[4][mm] * w[u + mm];
+      fv[f][u] = s;
+    }
+  }
+  const double ramp = __ldg(a.ramp + i);
+  double* out = a.coef + (long long)(j0 + row0) * P + i;
+#pragma unroll
+  for (int u = 0; u < NROW; ++u, out += P)
+    if ((on >> u) & 1u) zr_store(a, out, ramp, mu[u], fv[0][u], fv[1][u], fv[2][u]);
+}
+
+// The same for one point whose r row is not the centred one (closure row rw, or 9: blanked):
+// the 11 taps from the padded rows wt in shared memory, every load of a sum in flight.
+template <typename SIN, typename R>
+__device__ __forceinline__ void zr_closure_point(const ZrArgs& a, const double* zb, const SIN* tb, const double* wt,
+                                                 int rw, int p, int row, int i, int j0, int hr) {
+  const double mu = double(mu_k<R>(R(tb[row * ZRK_BZ + p])));
+  double fv[3] = {0.0, 0.0, 0.0};
+  if (rw < 9) {
+    const int w0 = tg_w0(rw);
+    const double* c0 = zb + p * ZRK_ZP + row + hr + w0;
+    double g[11];
+#pragma unroll
+    for (int mm = 0; mm < 11; ++mm) g[mm] = wt[rw * 21 + 10 + w0 + mm];
+#pragma unroll
+    for (int f = 0; f < 3; ++f) {
+      double x[11];
+#pragma unroll
+      for (int mm = 0; mm < 11; ++mm) x[mm] = c0[f * ZRK_BZ * ZRK_ZP + mm];
+      double s = g[0] * x[0];
+#pragma unroll
+      for (int mm = 1; mm < 11; ++mm) s = s + g[mm] * x[mm];
+      fv[f] = s;
+    }
+  }
+  zr_store(a, a.coef + (long long)(j0 + row) * a.g.P + i, __ldg(a.ramp + i), mu, fv[0], fv[1], fv[2]);
+}
+
+// The fused z/r filter of one CTA: z positions bx * a.seg .., the row block (j0, kind).
 template <typename SIN, typename R>
 __device__ __forceinline__ void zr_body(const ZrArgs& a, const CUtensorMap* pQ, const CUtensorMap* pZc,
-                                        const CUtensorMap* pRc, const CUtensorMap* pT, int bx, int by,
-                                        unsigned char* zrk_raw, uint64_t* bar) {
+                                        const CUtensorMap* pRc, const CUtensorMap* pT, int bx, int j0,
+                                        int kind, unsigned char* zrk_raw, uint64_t* bar) {
   using SM = ZrSmem<SIN>;
   unsigned char* base = zrk_raw + ((1024u - (smem_u32(zrk_raw) & 1023u)) & 1023u);
   double* wt = reinterpret_cast<double*>(base + SM::oW);
   const int tid = threadIdx.x;
   const int Nz = a.g.Nz, Nr = a.g.Nr;
-  const long long P = a.g.P, PL = a.g.plane;
+  const bool compact = kind & 1, closures = kind & 2;
+  const int hr = compact ? ZRK_HRC : ZRK_HRW;  // rows of the box below the block's first
   const int zs = bx * a.seg, ze = min(Nz, zs + a.seg);
-  const int j0 = by * ZRK_RB;
   const int bs = max(0, zs - ZRK_WARM) / ZRK_BZ;  // first block filtered (zs is a multiple of ZRK_BZ)
   const int be = (ze + ZRK_BZ - 1) / ZRK_BZ;       // blocks bs..be-1 are filtered, block be is loaded too
   // padded TG rows: row r's taps at offsets tg_w0(r) .. tg_w0(r) + tg_len(r) - 1 of
@@ -2094,10 +2231,10 @@ __device__ __forceinline__ void zr_body(const ZrArgs& a, const CUtensorMap* pQ, 
     const int sl = k & 1;
     unsigned char* q = base + SM::oQ + sl * SM::qslot;
     mbar_expect_tx(&bar[sl], SM::tx);
-    tma_load_3d(q, pQ, ZRK_BZ * k, j0 - ZRK_HR, 0, &bar[sl]);
-    tma_load_2d(base + SM::oZc + sl * 1024, pZc, ZRK_BZ * k, j0 - ZRK_HR, &bar[sl]);
+    tma_load_3d(q, pQ, ZRK_BZ * k, j0 - hr, 0, &bar[sl]);
+    tma_load_2d(base + SM::oZc + sl * 1024, pZc, ZRK_BZ * k, j0 - hr, &bar[sl]);
     tma_load_3d(base + SM::oT + sl * ((SM::tbytes + 127) / 128 * 128), pT, ZRK_BZ * (k - 1), j0, 4, &bar[sl]);
-    tma_load_2d(base + SM::oRc + sl * 512, pRc, ZRK_BZ * (k - 1), j0, &bar[sl]);
+    tma_load_2d(base + SM::oRc + sl * SM::rcslot, pRc, ZRK_BZ * (k - 1), j0, &bar[sl]);
   };
   if (tid == 0) issue(bs);
 
@@ -2105,10 +2242,8 @@ __device__ __forceinline__ void zr_body(const ZrArgs& a, const CUtensorMap* pQ, 
   const int fq = lane_on ? tid / ZRK_NR : 0;
   const int rr = lane_on ? tid - fq * ZRK_NR : 0;
   const int Rq = fq * ZRK_NR + rr;  // row of this recurrence in the Q / Z blocks
-  const int jr = j0 - ZRK_HR + rr;
+  const int jr = j0 - hr + rr;
   const bool row_on = lane_on && jr >= 0 && jr < Nr;
-  const double t0 = cTG[4][0], t1 = cTG[4][1], t2 = cTG[4][2], t3 = cTG[4][3], t4 = cTG[4][4];
-  const double t5 = cTG[4][5], t6 = cTG[4][6], t7 = cTG[4][7], t8 = cTG[4][8];
   double ring[16];  // filtered values, ring[p & 15] at position p
 #pragma unroll
   for (int k = 0; k < 16; ++k) ring[k] = 0.0;
@@ -2160,12 +2295,14 @@ __device__ __forceinline__ void zr_body(const ZrArgs& a, const CUtensorMap* pQ, 
       const bool centred = row_on && cws[0] == 0x04040404u && cws[1] == 0x04040404u && cws[2] == 0x04040404u &&
                            cws[3] == 0x04040404u && ZRK_BZ * m + ZRK_BZ <= Nz;
       if (centred) {
+        // the feed-forward sums first (independent of the recurrence and of each other), in
+        // place of the values no later step reads; then the feedback, a chain of one FMA of
+        // latency per step
 #pragma unroll
-        for (int s2 = 0; s2 < 16; ++s2) {
-          const double ff = t4 * xv[s2] + t5 * xv[s2 + 1] + t6 * xv[s2 + 2] + t7 * xv[s2 + 3] + t8 * xv[s2 + 4];
-          const double fb = t0 * ring[(s2 + 12) & 15] + t1 * ring[(s2 + 13) & 15] + t2 * ring[(s2 + 14) & 15];
-          ring[s2] = (ff + fb) + t3 * ring[(s2 + 15) & 15];
-        }
+        for (int s2 = 0; s2 < 16; ++s2) xv[s2] = zr_ff(xv[s2], xv[s2 + 1], xv[s2 + 2], xv[s2 + 3], xv[s2 + 4]);
+#pragma unroll
+        for (int s2 = 0; s2 < 16; ++s2)
+          ring[s2] = zr_fb(xv[s2], ring[(s2 + 12) & 15], ring[(s2 + 13) & 15], ring[(s2 + 14) & 15], ring[(s2 + 15) & 15]);
         double* zt = reinterpret_cast<double*>(zb) + fq * ZRK_BZ * ZRK_ZP + rr;
 #pragma unroll
         for (int s2 = 0; s2 < 16; ++s2) zt[s2 * ZRK_ZP] = ring[s2];
@@ -2178,21 +2315,23 @@ __device__ __forceinline__ void zr_body(const ZrArgs& a, const CUtensorMap* pQ, 
           if (p >= Nz) {
             v = 0.0;  // past the row: never stored, feeds only later positions past the row
           } else if (code == 4) {
-            // feed-forward and older feedback terms first, the newest filtered value last:
-            // one FMA of latency per step (the reference sums left to right; the orders
-            // differ by rounding only)
-            const double ff = t4 * xv[s2] + t5 * xv[s2 + 1] + t6 * xv[s2 + 2] + t7 * xv[s2 + 3] + t8 * xv[s2 + 4];
-            const double fb = t0 * ring[(s2 + 12) & 15] + t1 * ring[(s2 + 13) & 15] + t2 * ring[(s2 + 14) & 15];
-            v = (ff + fb) + t3 * ring[(s2 + 15) & 15];
+            v = zr_fb(zr_ff(xv[s2], xv[s2 + 1], xv[s2 + 2], xv[s2 + 3], xv[s2 + 4]), ring[(s2 + 12) & 15],
+                      ring[(s2 + 13) & 15], ring[(s2 + 14) & 15], ring[(s2 + 15) & 15]);
+          } else if (code >= 9) {
+            v = xv[s2];  // blanked (ModTGfilter.f90:18: the point keeps its value)
           } else {
-            // closure rows and blanked points: the padded 21-tap row, left to right
-            const double* w = wt + (code < 9 ? code : 9) * 21;
-            double acc = w[0] * ring[(s2 + 6) & 15];
+            // closure rows: the padded 21-tap row; the taps right of the point and the old
+            // feedback taps are independent sums, the newest filtered value comes last
+            const double* w = wt + code * 21;
+            double ff = w[10] * xv[s2], f2 = w[11] * xv[s2 + 1];
 #pragma unroll
-            for (int o = -9; o < 0; ++o) acc = acc + w[10 + o] * ring[(s2 + 16 + o) & 15];
+            for (int o = 2; o <= 10; o += 2) ff = ff + w[10 + o] * xv[s2 + o];
 #pragma unroll
-            for (int o = 0; o <= 10; ++o) acc = acc + w[10 + o] * xv[s2 + o];
-            v = acc;
+            for (int o = 3; o <= 9; o += 2) f2 = f2 + w[10 + o] * xv[s2 + o];
+            double fb = w[0] * ring[(s2 + 6) & 15];
+#pragma unroll
+            for (int o = -9; o < -1; ++o) fb = fb + w[10 + o] * ring[(s2 + 16 + o) & 15];
+            v = ((ff + f2) + fb) + w[9] * ring[(s2 + 15) & 15];
           }
           ring[s2] = v;
         }
@@ -2207,46 +2346,22 @@ __device__ __forceinline__ void zr_body(const ZrArgs& a, const CUtensorMap* pQ, 
     }
     __syncthreads();
     if (k > bs && ZRK_BZ * m + ZRK_BZ > zs) {
-      // r filter, scaling and coefficients of block m on the CTA's rows
+      // r filter, scaling and coefficients of block m on the CTA's rows: position tid % 16,
+      // ten groups of 4 (3) rows
       const SIN* tb = reinterpret_cast<const SIN*>(base + SM::oT + sl * ((SM::tbytes + 127) / 128 * 128));
-      const unsigned char* rcb = base + SM::oRc + sl * 512;
-      // the points of a thread are independent: unrolled so their T**0.666 and filter
-      // chains interleave
-#pragma unroll
-      for (int u = 0; u < (ZRK_RB * ZRK_BZ + ZRK_THREADS - 1) / ZRK_THREADS; ++u) {
-        const int qd = tid + u * ZRK_THREADS;
-        const int row = qd / ZRK_BZ, p = qd - row * ZRK_BZ;
-        const int j = j0 + row, i = ZRK_BZ * m + p;
-        if (qd >= ZRK_RB * ZRK_BZ || j >= Nr || i < zs || i >= ze) continue;
-        const double mu = double(mu_k<R>(R(tb[qd])));
-        const int rw = rcb[qd];
-        double fv[3] = {0.0, 0.0, 0.0};
-        // column of this point in the transposed block: row j0 + row is Z row row + ZRK_HR
-        const double* zc = reinterpret_cast<const double*>(zb) + p * ZRK_ZP + row + ZRK_HR;
-        if (rw == 4) {
-#pragma unroll
-          for (int f = 0; f < 3; ++f) {
-            const double* col = zc + f * ZRK_BZ * ZRK_ZP - 4;
-            double sacc = t0 * col[0];
-#pragma unroll
-            for (int mm = 1; mm < 9; ++mm) sacc = sacc + cTG[4][mm] * col[mm];
-            fv[f] = sacc;
-          }
-        } else if (rw < 9) {
-          const int w0 = tg_w0(rw), n = tg_len(rw);
-#pragma unroll
-          for (int f = 0; f < 3; ++f) {
-            const double* col = zc + f * ZRK_BZ * ZRK_ZP + w0;
-            double sacc = cTG[rw][0] * col[0];
-            for (int mm = 1; mm < n; ++mm) sacc = sacc + cTG[rw][mm] * col[mm];
-            fv[f] = sacc;
+      const unsigned char* rcb = base + SM::oRc + sl * SM::rcslot;
+      const int p = tid & (ZRK_BZ - 1), g = tid / ZRK_BZ, i = ZRK_BZ * m + p;
+      const double* zd = reinterpret_cast<const double*>(zb);
+      if (i >= zs && i < ze) {
+        if (compact) zr_points<ZRK_RBC / 10, SIN, R>(a, zd, tb, rcb, p, g * (ZRK_RBC / 10), i, j0, hr);
+        else zr_points<ZRK_RBW / 10, SIN, R>(a, zd, tb, rcb, p, g * (ZRK_RBW / 10), i, j0, hr);
+        if (closures) {
+          const int nr = min(compact ? ZRK_RBC : ZRK_RBW, Nr - j0);
+          for (int row = g; row < nr; row += ZRK_THREADS / ZRK_BZ) {
+            const int rw = rcb[row * ZRK_BZ + p];
+            if (rw != 4) zr_closure_point<SIN, R>(a, zd, tb, wt, rw, p, row, i, j0, hr);
           }
         }
-        const double ramp = __ldg(a.ramp + i);
-        const long long o = (long long)j * P + i;
-        a.coef[o] = mu + a.c.C_mu_Re * fv[0] * ramp;
-        a.coef[PL + o] = (3.0 / 5.0) * mu + a.c.C_beta_Re * fv[1] * ramp;
-        a.coef[2 * PL + o] = mu + a.c.C_kappa_Re_Pr * fv[2] * ramp;
       }
     }
     __syncthreads();
@@ -2259,10 +2374,11 @@ __global__ void __launch_bounds__(ZRK_THREADS, 3)
               const __grid_constant__ CUtensorMap mRc, const __grid_constant__ CUtensorMap mT) {
   extern __shared__ __align__(128) unsigned char zrk_raw[];
   __shared__ __align__(8) uint64_t bar[2];
-  zr_body<SIN, R>(a, &mQ, &mZc, &mRc, &mT, blockIdx.x, blockIdx.y, zrk_raw, bar);
+  const int2 rb = a.rblocks[blockIdx.y];
+  zr_body<SIN, R>(a, &mQ, &mZc, &mRc, &mT, blockIdx.x, rb.x, rb.y, zrk_raw, bar);
 }
 
-// Batched: one CTA per entry (segment, row block, instance) of a table over all instances;
+// Batched: one CTA per entry (segment, first row, instance, kind) of a table over all instances;
 // each instance's arguments (staged in shared memory) and maps come from device tables.
 template <typename SIN, typename R>
 __global__ void __launch_bounds__(ZRK_THREADS, 3)
@@ -2276,12 +2392,12 @@ __global__ void __launch_bounds__(ZRK_THREADS, 3)
     reinterpret_cast<unsigned long long*>(&sa)[k] = reinterpret_cast<const unsigned long long*>(argv + it.z)[k];
   __syncthreads();
   const CUtensorMap* m = mapv + (size_t)it.z * nmaps;
-  zr_body<SIN, R>(sa, m + kmaps.x, m + kmaps.y, m + kmaps.z, m + kmaps.w, it.x, it.y, zrk_raw, bar);
+  zr_body<SIN, R>(sa, m + kmaps.x, m + kmaps.y, m + kmaps.z, m + kmaps.w, it.x, it.y, it.w, zrk_raw, bar);
 }
 
 template <typename SIN, typename R>
 static cudaError_t launch_zr_t(const ZrArgs& a, const ZrMaps& m, cudaStream_t s) {
-  const dim3 grid((a.g.Nz + a.seg - 1) / a.seg, (a.g.Nr + ZRK_RB - 1) / ZRK_RB);
+  const dim3 grid((a.g.Nz + a.seg - 1) / a.seg, a.nrblocks);
   zr_kernel<SIN, R><<<grid, ZRK_THREADS, ZrSmem<SIN>::bytes, s>>>(a, *m.q, *m.zc, *m.rc, *m.t);
   return cudaGetLastError();
 }

@@ -168,23 +168,31 @@ cudaError_t launch_sensor_tiles_only(const SensorArgs& a, const SideStream& side
 
 // Fused z filter + r filter + transport coefficients (zr_kernel): from Q to the planes
 // mu_eff, beta = 0.6 mu + beta*, kappa_eff of the stage input. A CTA of ZRK_THREADS
-// threads owns seg z positions (a multiple of ZRK_BZ) and ZRK_RB rows.
+// threads owns seg z positions (a multiple of ZRK_BZ) and one row block.
 constexpr int ZRK_BZ = 16;                    // z positions per block (one 128-byte row of doubles)
-constexpr int ZRK_RB = 30;                    // rows per CTA (30 x 16 points: three per thread)
-constexpr int ZRK_HR = 10;                    // r reach of the TG boundary rows
-constexpr int ZRK_NR = ZRK_RB + 2 * ZRK_HR;   // rows of the z recurrence per CTA
+constexpr int ZRK_NR = 50;                    // rows of the z recurrence per CTA (3 x 50 of its threads)
 constexpr int ZRK_THREADS = 160;
+// Row blocks: a CTA owns the middle rows of its ZRK_NR. The r filter's centred row reaches 4
+// rows, its 11-point boundary rows up to 10, but on one side: a compact block owns 40 rows
+// (1.25 recurrences per row) and serves wherever every window of its rows stays within 5 rows
+// of it, which holds at r = 0 and r = r_max too (their windows lie inside); a wide block owns
+// 30 rows (1.67) and serves anywhere.
+constexpr int ZRK_RBC = 40, ZRK_HRC = 5;      // compact
+constexpr int ZRK_RBW = 30, ZRK_HRW = 10;     // wide
+constexpr int ZRK_WARM = 48;                  // warm-up positions of a segment (3 blocks)
 struct ZrArgs {
   Grid g;
   const double* ramp;  // (1+tanh(5(z-10)))/2 per i
   double* coef;        // 3 planes: mu_eff, beta, kappa_eff
   int* flags;          // bit 2: a bounded wait gave up
+  const int2* rblocks; // row blocks (first row, kind: bit 0 compact, bit 1 holds rows that are not centred)
+  int nrblocks;
   int seg;             // z positions per CTA (multiple of ZRK_BZ)
   Consts c;
 };
 // TMA maps: q = Q (3 planes of doubles, box {ZRK_BZ, ZRK_NR, 3}, 128-byte swizzle);
-// zc / rc = z / r row codes (uint8, 9 = blanked; boxes {ZRK_BZ, ZRK_NR} / {ZRK_BZ, ZRK_RB});
-// t = the stage input's planes (box {ZRK_BZ, ZRK_RB, 1}, FP32 when in_f32).
+// zc / rc = z / r row codes (uint8, 9 = blanked; boxes {ZRK_BZ, ZRK_NR} / {ZRK_BZ, ZRK_RBC});
+// t = the stage input's planes (box {ZRK_BZ, ZRK_RBC, 1}, FP32 when in_f32).
 struct ZrMaps {
   const CUtensorMap* q;
   const CUtensorMap* zc;
@@ -192,7 +200,7 @@ struct ZrMaps {
   const CUtensorMap* t;
 };
 cudaError_t launch_zr(const ZrArgs& a, const ZrMaps& m, bool mixed, bool in_f32, cudaStream_t s);
-// Batched fused z/r filter: items (segment, row block, instance, 0), per-instance arguments
+// Batched fused z/r filter: items (segment, first row, instance, kind of the row block), per-instance arguments
 // and the maps of the batch table (kin = stage-input buffer id).
 cudaError_t launch_zr_batch(const ZrArgs* argv, const int4* items, int nitems, const CUtensorMap* mapv, int kin,
                             bool mixed, bool in_f32, cudaStream_t s);

@@ -35,7 +35,7 @@ constexpr int NA_BAD = NA_MAX_BLOCKS + 1;             // slot of the non-finite 
 static __device__ __align__(256) double g_dt_scratch[NA_MAX_BLOCKS + 2];
 // the tables of the FP64 power mu = T**0.666 (axj_pow.cuh), written by the first call on
 // each device
-static __device__ double g_na_pow[axj::POW_TAB];
+static __device__ __align__(16) double g_na_pow[axj::POW_TAB];
 
 __device__ __forceinline__ double na_warp_min(double v) {
 #pragma unroll
