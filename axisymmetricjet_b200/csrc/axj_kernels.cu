@@ -48,14 +48,16 @@ __device__ __forceinline__ R mu_k(R T) {
 
 // mu of N stage inputs; in FP64 without a branch between them (their table loads and chains
 // interleave), the rare T outside the tables' range afterwards.
-template <int N, typename R>
+// ZERO: T = 0 (a halo never written) gives 0 without leaving the fast path.
+template <int N, typename R, bool ZERO = false>
 __device__ __forceinline__ void mu_n(const R (&T)[N], double (&mu)[N]) {
   if constexpr (std::is_same<R, double>::value) {
     bool ok = true;
 #pragma unroll
     for (int u = 0; u < N; ++u) {
       mu[u] = pow0666_table(T[u], gPowTab);
-      ok = ok && pow0666_in_range(T[u]);
+      if (ZERO && T[u] == 0.0) mu[u] = 0.0;
+      else ok = ok && pow0666_in_range(T[u]);
     }
     if (!ok) {
 #pragma unroll 1
@@ -174,6 +176,65 @@ __device__ __forceinline__ R dst_p(int row, const S* rho, const S* T, int stride
     s = s + tabv<R, 1>(rw, m) * (R(rho[(w0 + m) * stride]) * R(T[(w0 + m) * stride]));
   }
   return s;
+}
+
+// A stencil row as six taps (general tiles): the weights of both operators, the window's start
+// and the sixth tap's offset. Every row fits: the centred row's sixth weight is zero (that tap
+// reads the point itself), row 9 (no derivative) has zero weights. Read from a table in shared
+// memory [ROW6_ROWS][12], so lanes of a warp with different rows take one path.
+constexpr int ROW6_ROWS = 10;
+template <typename R>
+struct Row6 {
+  R a[6], b[6];  // SBP1, SBP2
+  int w0, o5;
+};
+template <typename R>
+__device__ __forceinline__ void row6_fill(R* tab, int tid, int nt) {
+  for (int e = tid; e < ROW6_ROWS * 12; e += nt) {
+    const int r = e / 12, k = e - 12 * r, m = k % 6;
+    tab[e] = r < 9 ? (k < 6 ? tabv<R, 1>(r, m) : tabv<R, 2>(r, m)) : R(0);
+  }
+}
+template <typename R>
+__device__ __forceinline__ Row6<R> row6(const R* tab, int row) {
+  Row6<R> q;
+  const R* t = tab + 12 * min(row, 9);
+#pragma unroll
+  for (int m = 0; m < 6; ++m) {
+    q.a[m] = t[m];
+    q.b[m] = t[6 + m];
+  }
+  q.w0 = row < 9 ? sbp_w0(row) : 0;
+  q.o5 = row == 4 || row >= 9 ? 0 : q.w0 + 5;
+  if (row >= 9) q.w0 = -2;  // zero weights on the centred window
+  return q;
+}
+// First (D = 1) or second derivative at p by the centred row (C) or by q, taps left to right.
+template <typename R, bool C, int D, typename S>
+__device__ __forceinline__ R dst6(const Row6<R>& q, const S* p, int stride) {
+  if constexpr (C) {
+    if constexpr (D == 1) return dot_c1<R>(p, stride);
+    else return dotc<R, 2, 5>(4, p - 2 * stride, stride);
+  } else {
+    const R* w = D == 1 ? q.a : q.b;
+    const S* v = p + q.w0 * stride;
+    R s = w[0] * R(v[0]);
+#pragma unroll
+    for (int m = 1; m < 5; ++m) s = s + w[m] * R(v[m * stride]);
+    return s + w[5] * R(p[q.o5 * stride]);
+  }
+}
+template <typename R, bool C, typename S>
+__device__ __forceinline__ R dst6_p(const Row6<R>& q, const S* rho, const S* T, int stride) {
+  if constexpr (C) {
+    return dst_p<R, false>(4, rho, T, stride);
+  } else {
+    const S *a = rho + q.w0 * stride, *b = T + q.w0 * stride;
+    R s = q.a[0] * (R(a[0]) * R(b[0]));
+#pragma unroll
+    for (int m = 1; m < 5; ++m) s = s + q.a[m] * (R(a[m * stride]) * R(b[m * stride]));
+    return s + q.a[5] * (R(rho[q.o5 * stride]) * R(T[q.o5 * stride]));
+  }
 }
 
 // 9-point fourth difference cC9 centred at p (stride in elements), left to right.
@@ -319,13 +380,22 @@ struct StageSmem {
     return align128(oDesc(gen) + (gen ? sizeof(uint32_t) * NPT : 0));
   }
   static constexpr int NMET = 3 * TZ + 4 * TRT;
-  __host__ __device__ static constexpr size_t bytes(bool gen) { return align128(oMet(gen) + sizeof(double) * NMET); }
+  // general tiles: the six-tap stencil rows
+  __host__ __device__ static constexpr size_t oRow(bool gen) { return align128(oMet(gen) + sizeof(double) * NMET); }
+  __host__ __device__ static constexpr size_t bytes(bool gen) {
+    return align128(oRow(gen) + (gen ? sizeof(R) * ROW6_ROWS * 12 : 0));
+  }
   static constexpr uint32_t state_bytes = sizeof(SIN) * 5 * NPT;
   static constexpr uint32_t q_bytes = sizeof(double) * 3 * RQ * RZ;
   static constexpr uint32_t tile_bytes = sizeof(double) * 5 * NTP;
   static constexpr int NPER = (NPT + STAGE_THREADS - 1) / STAGE_THREADS;
 };
 
+
+// What bounds the general tiles is one tile's latency (few tiles, closure rows). Measured on a
+// B200 when their loads of the RK operands, descriptors and stencil rows were grouped and the
+// stencils made branch-free (below): 96 x 64 16.7 -> 13.3 us per stage, 512 x 128 18.3 -> 14.7,
+// 4400 x 640 24.9 -> 20.3; a batch of 12 jets (mixed) 113 -> 63 us.
 
 // Fused RK stage. SIN: storage type of the stage input (double, or float for the
 // mixed path's intermediate stages); R: arithmetic type of the stencils and, in
@@ -343,6 +413,7 @@ struct StagePtrs {
   R* sDz;
   const uint32_t* sDesc;
   const double* sMet;
+  const R* sRow;  // six-tap stencil rows (general tiles)
 };
 
 // Phases 2-3 of one stage tile (i0, j0; nrow rows of it are owned) whose boxes have
@@ -368,14 +439,18 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
   R* sDz = sp.sDz;
   const uint32_t* sDesc = sp.sDesc;
   const double* sMet = sp.sMet;
+  const R* sRow = sp.sRow;
   const int tid = threadIdx.x;
   const int Nz = a.g.Nz, Nr = a.g.Nr;
   const long long P = a.g.P, PL = a.g.plane;
   const bool sc = a.c.shock_capturing != 0;
   // RK operands from global memory (general tiles, FP32 half tiles) or staged by TMA
   constexpr bool RKG = GEN || rk_global<R, TRT>();
-  const bool needU0 = !RKG && (a.stage == 2 || a.stage == 3);
-  const bool needA = !RKG && (a.stage == 3 || a.stage == 4);
+  // a double stage input with FP32 stencils is the mixed path's pv: stage 1, or the right-hand
+  // side alone (stage 0); the later stages' code is left out of those instances
+  constexpr bool FIRST = !std::is_same<SIN, R>::value;
+  const bool needU0 = !FIRST && !RKG && (a.stage == 2 || a.stage == 3);
+  const bool needA = !FIRST && !RKG && (a.stage == 3 || a.stage == 4);
   // mu = T**0.666 (AssignValues) on the cross of the region (CM_PRE: the coefficient box
   // already holds mu_eff, beta and kappa_eff). With shock capturing the
   // coefficient box holds the z-filtered quantities; the r filter PerformTGfilter(q, 2,
@@ -386,16 +461,22 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
   // mu = 0, as the never-written halo does; blanked points keep mu* = 0.
   if (CM != CM_PRE) {
     double vmu[NPER], vbe[NPER], vka[NPER];
+    {
+      // (every point's power, the region's corners too: without branches they interleave)
+      R T[NPER];
+#pragma unroll
+      for (int k = 0; k < NPER; ++k) T[k] = R(sU[4 * NPT + min(tid + k * NT, NPT - 1)]);
+      mu_n<NPER, R, true>(T, vmu);
+    }
 #pragma unroll
     for (int k = 0; k < NPER; ++k) {
       const int idx = tid + k * NT;
-      vmu[k] = vbe[k] = vka[k] = 0.0;
+      const double mu = vmu[k];
+      vbe[k] = vka[k] = 0.0;
       if (idx >= NPT) continue;
       const int rr = idx / RZ, rz = idx - rr * RZ;
       const bool cross = (rr >= H && rr < H + TRT && rz >= HZ - H && rz < HZ + TZ + H) || (rz >= HZ && rz < HZ + TZ);
       if (!cross) continue;
-      const double mu = double(mu_k<R>(R(sU[4 * NPT + idx])));
-      vmu[k] = mu;
       if (rr >= H && rr < H + TRT && rz >= HZ && rz < HZ + TZ) sMu0[(rr - H) * TZ + (rz - HZ)] = mu;
       if (sc) {
         int rw = 4;
@@ -455,21 +536,34 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
 
   // ---- phase 2: dVr/dz and dVz/dz on the tile columns, all region rows (needed by
   // the mixed derivatives d/dr(dV/dz), ModRHS.f90:132-133)
-  for (int idx = tid; idx < RR * TZ; idx += NT) {
+  // (a warp takes one row of the region; its passes are unrolled, so that their loads overlap)
+  static_assert(TZ == 32 && NT % TZ == 0, "a warp per region row");
+#pragma unroll
+  for (int q = 0; q < (RR * TZ + NT - 1) / NT; ++q) {
+    const int idx = tid + q * NT;
+    if (RR * TZ % NT != 0 && idx >= RR * TZ) break;  // whole warps
     const int rr = idx / TZ, c = idx - rr * TZ;
     const int i = i0 + c, j = j0 - H + rr;
-    R dvr = R(0), dvz = R(0);
-    const bool in = (!GEN) || (i < Nz && j >= 0 && j < Nr);
-    if (in) {
-      const int sidx = rr * RZ + HZ + c;
-      int row = 4;
-      if (GEN) {
+    const int sidx = rr * RZ + HZ + c;
+    const R m = R(sMet[c]);
+    R dvr, dvz;
+    if constexpr (GEN) {
+      int row = (int)ROW_NONE;
+      if (i < Nz && j >= 0 && j < Nr) {
         const uint32_t dsc = sDesc[sidx];
         row = desc_blank(dsc) ? (int)ROW_NONE : desc_zrow(dsc);
       }
-      const R m = R(sMet[c]);
-      dvr = dst<R, 1, GEN>(row, sU + 1 * NPT + sidx, 1) * m;
-      dvz = dst<R, 1, GEN>(row, sU + 3 * NPT + sidx, 1) * m;
+      if (__all_sync(0xffffffffu, row == 4)) {
+        dvr = dot_c1<R>(sU + 1 * NPT + sidx, 1) * m;
+        dvz = dot_c1<R>(sU + 3 * NPT + sidx, 1) * m;
+      } else {
+        const Row6<R> w = row6(sRow, row);
+        dvr = row < 9 ? dst6<R, false, 1>(w, sU + 1 * NPT + sidx, 1) * m : R(0);
+        dvz = row < 9 ? dst6<R, false, 1>(w, sU + 3 * NPT + sidx, 1) * m : R(0);
+      }
+    } else {
+      dvr = dot_c1<R>(sU + 1 * NPT + sidx, 1) * m;
+      dvz = dot_c1<R>(sU + 3 * NPT + sidx, 1) * m;
     }
     sDz[idx] = dvr;
     sDz[RR * TZ + idx] = dvz;
@@ -490,18 +584,22 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
   for (int pidx = tid; pidx < TZ * TRT; pidx += NT) {
     const int r = pidx / TZ, c = pidx - r * TZ;
     const int i = i0 + c, j = j0 + r;
-    if (GEN && (i >= Nz || j >= Nr || r >= nrow)) continue;
+    if (GEN && (j >= Nr || r >= nrow)) break;  // whole warps (a row each), rows ascending
     const int rr = H + r, rz = HZ + c;
     const int sidx = rr * RZ + rz;
     int zr = 4, rw = 4;
     bool blank = false;
     uint32_t face = 0;
+    bool z4 = true, r4 = true;  // every point of the warp has the centred row
     if (GEN) {
       const uint32_t dsc = sDesc[sidx];
       blank = desc_blank(dsc);
       zr = blank ? (int)ROW_NONE : desc_zrow(dsc);
       rw = blank ? (int)ROW_NONE : desc_rrow(dsc);
       face = desc_face(dsc);
+      z4 = __all_sync(0xffffffffu, i >= Nz || zr == 4);
+      r4 = __all_sync(0xffffffffu, i >= Nz || rw == 4);
+      if (i >= Nz) continue;
     }
     const double xzd = sMet[c], erd = sMet[3 * TZ + r];
     const R xz = R(xzd), xzz = R(sMet[TZ + c]);
@@ -516,34 +614,55 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
     const int dzi = rr * TZ + c;
 
     DerivT<R> dr;
-    // first derivatives (Compute1stDerivative: stencil, then * metric)
-    dr.drhodz = dst<R, 1, GEN>(zr, pR, 1) * xz;
-    dr.dVrdz = sDz[dzi];
-    dr.dVtdz = dst<R, 1, GEN>(zr, pVt, 1) * xz;
-    dr.dVzdz = sDz[RR * TZ + dzi];
-    dr.dTdz = dst<R, 1, GEN>(zr, pT, 1) * xz;
-    dr.dpdz = dst_p<R, GEN>(zr, pR, pT, 1) * xz;
-    dr.drhodr = dst<R, 1, GEN>(rw, pR, RZ) * er;
-    dr.dVrdr = dst<R, 1, GEN>(rw, pVr, RZ) * er;
-    dr.dVtdr = dst<R, 1, GEN>(rw, pVt, RZ) * er;
-    dr.dVzdr = dst<R, 1, GEN>(rw, pVz, RZ) * er;
-    dr.dTdr = dst<R, 1, GEN>(rw, pT, RZ) * er;
-    dr.dpdr = dst_p<R, GEN>(rw, pR, pT, RZ) * er;
-    // second derivatives (Compute2ndDerivative: out*metric**2 + f'*metric')
-    dr.d2Vrdz2 = dst<R, 2, GEN>(zr, pVr, 1) * (xz * xz) + dr.dVrdz * xzz;
-    dr.d2Vtdz2 = dst<R, 2, GEN>(zr, pVt, 1) * (xz * xz) + dr.dVtdz * xzz;
-    dr.d2Vzdz2 = dst<R, 2, GEN>(zr, pVz, 1) * (xz * xz) + dr.dVzdz * xzz;
-    dr.d2Tdz2 = dst<R, 2, GEN>(zr, pT, 1) * (xz * xz) + dr.dTdz * xzz;
-    dr.d2Vrdr2 = dst<R, 2, GEN>(rw, pVr, RZ) * (er * er) + dr.dVrdr * err;
-    dr.d2Vtdr2 = dst<R, 2, GEN>(rw, pVt, RZ) * (er * er) + dr.dVtdr * err;
-    dr.d2Vzdr2 = dst<R, 2, GEN>(rw, pVz, RZ) * (er * er) + dr.dVzdr * err;
-    dr.d2Tdr2 = dst<R, 2, GEN>(rw, pT, RZ) * (er * er) + dr.dTdr * err;
-    dr.dmudz = dst<R, 1, GEN>(zr, pMu, 1) * xz;
-    dr.dkappadz = sc ? dst<R, 1, GEN>(zr, pKa, 1) * xz : dr.dmudz;
-    dr.dmudr = dst<R, 1, GEN>(rw, pMu, RZ) * er;
-    dr.dkappadr = sc ? dst<R, 1, GEN>(rw, pKa, RZ) * er : dr.dmudr;
-    dr.d2Vrdzdr = dst<R, 1, GEN>(rw, sDz + dzi, TZ) * er;
-    dr.d2Vzdzdr = dst<R, 1, GEN>(rw, sDz + RR * TZ + dzi, TZ) * er;
+    // first derivatives (Compute1stDerivative: stencil, then * metric) and second derivatives
+    // (Compute2ndDerivative: out*metric**2 + f'*metric'). General tiles branch once per warp and
+    // direction, between the centred row and the six-tap form of any row: with a branch in
+    // every derivative, the 26 stencils neither shared their loads nor overlapped.
+    auto along_z = [&](auto centred) {
+      constexpr bool C = decltype(centred)::value;
+      Row6<R> q;
+      if constexpr (!C) q = row6(sRow, zr);
+      dr.drhodz = dst6<R, C, 1>(q, pR, 1) * xz;
+      dr.dVrdz = sDz[dzi];
+      dr.dVtdz = dst6<R, C, 1>(q, pVt, 1) * xz;
+      dr.dVzdz = sDz[RR * TZ + dzi];
+      dr.dTdz = dst6<R, C, 1>(q, pT, 1) * xz;
+      dr.dpdz = dst6_p<R, C>(q, pR, pT, 1) * xz;
+      dr.d2Vrdz2 = dst6<R, C, 2>(q, pVr, 1) * (xz * xz) + dr.dVrdz * xzz;
+      dr.d2Vtdz2 = dst6<R, C, 2>(q, pVt, 1) * (xz * xz) + dr.dVtdz * xzz;
+      dr.d2Vzdz2 = dst6<R, C, 2>(q, pVz, 1) * (xz * xz) + dr.dVzdz * xzz;
+      dr.d2Tdz2 = dst6<R, C, 2>(q, pT, 1) * (xz * xz) + dr.dTdz * xzz;
+      dr.dmudz = dst6<R, C, 1>(q, pMu, 1) * xz;
+      dr.dkappadz = sc ? dst6<R, C, 1>(q, pKa, 1) * xz : dr.dmudz;
+    };
+    auto along_r = [&](auto centred) {
+      constexpr bool C = decltype(centred)::value;
+      Row6<R> q;
+      if constexpr (!C) q = row6(sRow, rw);
+      dr.drhodr = dst6<R, C, 1>(q, pR, RZ) * er;
+      dr.dVrdr = dst6<R, C, 1>(q, pVr, RZ) * er;
+      dr.dVtdr = dst6<R, C, 1>(q, pVt, RZ) * er;
+      dr.dVzdr = dst6<R, C, 1>(q, pVz, RZ) * er;
+      dr.dTdr = dst6<R, C, 1>(q, pT, RZ) * er;
+      dr.dpdr = dst6_p<R, C>(q, pR, pT, RZ) * er;
+      dr.d2Vrdr2 = dst6<R, C, 2>(q, pVr, RZ) * (er * er) + dr.dVrdr * err;
+      dr.d2Vtdr2 = dst6<R, C, 2>(q, pVt, RZ) * (er * er) + dr.dVtdr * err;
+      dr.d2Vzdr2 = dst6<R, C, 2>(q, pVz, RZ) * (er * er) + dr.dVzdr * err;
+      dr.d2Tdr2 = dst6<R, C, 2>(q, pT, RZ) * (er * er) + dr.dTdr * err;
+      dr.dmudr = dst6<R, C, 1>(q, pMu, RZ) * er;
+      dr.dkappadr = sc ? dst6<R, C, 1>(q, pKa, RZ) * er : dr.dmudr;
+      dr.d2Vrdzdr = dst6<R, C, 1>(q, sDz + dzi, TZ) * er;
+      dr.d2Vzdzdr = dst6<R, C, 1>(q, sDz + RR * TZ + dzi, TZ) * er;
+    };
+    if constexpr (GEN) {
+      if (z4) along_z(std::true_type{});
+      else along_z(std::false_type{});
+      if (r4) along_r(std::true_type{});
+      else along_r(std::false_type{});
+    } else {
+      along_z(std::true_type{});
+      along_r(std::true_type{});
+    }
 
     const double pv[5] = {double(*pR), double(*pVr), double(*pVt), double(*pVz), double(*pT)};
     PrimT<RP> q;
@@ -578,6 +697,20 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
 #pragma unroll
       for (int f = 0; f < 5; ++f) rhs[f] = double(rp[f]);
     }
+    // the RK update's operands: all their loads together and ahead of the face operations (one
+    // field after the other, each load waits behind the previous field's store to A or B, which
+    // it might alias: five memory latencies in a row)
+    const int tp = r * TZ + c;  // index in the tile boxes
+    double u0v[5], av[5], bv[5];
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+      const long long o = f * PL + go;
+      u0v[f] = av[f] = bv[f] = 0.0;
+      if (FIRST) continue;
+      if (a.stage == 2 || a.stage == 3) u0v[f] = RKG ? __ldg(a.U0 + o) : sP0[f * NTP + tp];
+      if (a.stage == 3 || a.stage == 4) av[f] = RKG ? a.A[o] : sPA[f * NTP + tp];
+      if (a.stage == 3) bv[f] = __ldg(a.B + o);
+    }
     // pv_target is read only where a term uses it: sponges, face operations, forcing
     const bool need_tg = (rloc >= a.c.sponge_start_top) || (!j1 && zloc <= a.c.sponge_end_left) ||
                          a.c.control_forcing == 1 || (GEN && face);
@@ -606,26 +739,23 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
     }
     // ---- RK4 stage update (ModRungeKutta.f90:32-51, :134-146), always in double
     const double c6 = 1.0 / 6.0, c3 = 1.0 / 3.0;
-    const int tp = r * TZ + c;  // index in the tile boxes
     double un[5];
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
       const double k = mul_rn(dtv, rhs[f]);
       const long long o = f * PL + go;
-      if (a.stage == 1) {
+      if (FIRST || a.stage == 1) {
         const double u0 = pv[f];  // pv_old = stage-1 input
         un[f] = add_rn(u0, mul_rn(0.5, k));
         a.A[o] = add_rn(u0, mul_rn(c6, k));
       } else if (a.stage == 2) {
-        const double u0 = RKG ? __ldg(a.U0 + o) : sP0[f * NTP + tp];
-        un[f] = add_rn(u0, mul_rn(0.5, k));
+        un[f] = add_rn(u0v[f], mul_rn(0.5, k));
         a.B[o] = k;
       } else if (a.stage == 3) {
-        const double u0 = RKG ? __ldg(a.U0 + o) : sP0[f * NTP + tp];
-        un[f] = add_rn(u0, k);
-        a.A[o] = add_rn(RKG ? a.A[o] : sPA[f * NTP + tp], mul_rn(c3, add_rn(__ldg(a.B + o), k)));
+        un[f] = add_rn(u0v[f], k);
+        a.A[o] = add_rn(av[f], mul_rn(c3, add_rn(bv[f], k)));
       } else {
-        un[f] = blank ? pv[f] : add_rn(RKG ? a.A[o] : sPA[f * NTP + tp], mul_rn(c6, k));
+        un[f] = blank ? pv[f] : add_rn(av[f], mul_rn(c6, k));
       }
     }
     if (j1) {
@@ -635,14 +765,14 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       un[3] = axis_extrap(pVz + RZ, RZ);
       un[4] = axis_extrap(pT + RZ, RZ);
     }
-    if (a.out_f32 && a.stage < 4) {
+    if (FIRST || (a.out_f32 && a.stage < 4)) {
 #pragma unroll
       for (int f = 0; f < 5; ++f) a.Uout_f[f * PL + go] = float(un[f]);
     } else {
 #pragma unroll
       for (int f = 0; f < 5; ++f) a.Uout[f * PL + go] = un[f];
     }
-    if (a.stage == 4) {
+    if (!FIRST && a.stage == 4) {
       bool bad = false;
 #pragma unroll
       for (int f = 0; f < 5; ++f) bad |= !isfinite(un[f]);
@@ -670,6 +800,7 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
   R* sDz = reinterpret_cast<R*>(smem_raw + SM::oDz(GEN));         // [2][RR][TZ]
   uint32_t* sDesc = reinterpret_cast<uint32_t*>(smem_raw + SM::oDesc(GEN));
   double* sMet = reinterpret_cast<double*>(smem_raw + SM::oMet(GEN));  // [3][TZ] + [4][TR]
+  R* sRow = reinterpret_cast<R*>(smem_raw + SM::oRow(GEN));            // [ROW6_ROWS][12]
 
   const int tid = threadIdx.x;
   const int Nz = a.g.Nz, Nr = a.g.Nr;
@@ -717,14 +848,6 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
     if (RKG && (a.stage == 2 || a.stage == 3)) tma_prefetch_3d(mU0, i0, j0, 0);
     if (RKG && (a.stage == 3 || a.stage == 4)) tma_prefetch_3d(mAcc, i0, j0, 0);
   }
-  if (GEN) {
-    for (int idx = tid; idx < NPT; idx += NT) {
-      const int rr = idx / RZ, rz = idx - rr * RZ;
-      const int i = i0 - HZ + rz, j = j0 - H + rr;
-      sDesc[idx] = (i >= 0 && i < Nz && j >= 0 && j < Nr) ? __ldg(a.desc + (long long)j * P + i)
-                                                            : make_desc(ROW_NONE, ROW_NONE, false, 0);
-    }
-  }
   // the tile's metrics and coordinates (read per point in phases 2-3)
   if (tid < TZ) {
     const int i = min(i0 + tid, Nz - 1);
@@ -738,6 +861,23 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
     sMet[3 * TZ + 2 * TRT + r] = __ldg(a.rc + j);
     sMet[3 * TZ + 3 * TRT + r] = __ldg(a.invr + j);
   }
+  if constexpr (GEN) {
+    // the region's descriptors, all of a thread's loads in flight
+    constexpr int ND = (NPT + NT - 1) / NT;
+    uint32_t dv[ND];
+#pragma unroll
+    for (int q = 0; q < ND; ++q) {
+      const int idx = tid + q * NT;
+      const int rr = idx / RZ, rz = idx - rr * RZ;
+      const int i = i0 - HZ + rz, j = j0 - H + rr;
+      dv[q] = (idx < NPT && i >= 0 && i < Nz && j >= 0 && j < Nr) ? __ldg(a.desc + (long long)j * P + i)
+                                                                  : make_desc(ROW_NONE, ROW_NONE, false, 0);
+    }
+    row6_fill(sRow, tid, NT);
+#pragma unroll
+    for (int q = 0; q < ND; ++q)
+      if (tid + q * NT < NPT) sDesc[tid + q * NT] = dv[q];
+  }
   if (!__syncthreads_and(mbar_wait_bounded(&bar[0], phase & 1u))) {
     if (tid == 0) atomicOr(a.flags, 4);
     mbar_drain(&bar[0], phase & 1u);
@@ -745,7 +885,7 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
     return false;
   }
   phase ^= 1u;
-  const StagePtrs<SIN, R> sp{sU, sQ, sMu0, sP0, sPA, sDz, sDesc, sMet};
+  const StagePtrs<SIN, R> sp{sU, sQ, sMu0, sP0, sPA, sDz, sDesc, sMet, sRow};
   const bool ok = stage_compute<H, GEN, SIN, R, CM, NT, TRT>(a, i0, j0, nrow, sp, &bar[1], (phase >> 1) & 1u);
   if (ok && (needU0 || needA)) phase ^= 2u;
   return ok;
@@ -756,19 +896,29 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
 // Threads of a stage CTA: 256 for tiles of TR rows (two CTAs per SM), 128 for the half
 // tiles of TR / 2 rows (four CTAs per SM, six with FP32 stencils: while one waits for its
 // boxes, the others compute).
-__host__ __device__ constexpr int stage_threads(int trt) { return trt == TR ? STAGE_THREADS : STAGE_THREADS / 2; }
+// General tiles take 512 threads (WIDE: one point per thread, one CTA per SM) where there is at
+// most one of them per SM: the kernel's time is then one tile's latency, which two points per
+// thread double (512 x 128, 46 tiles: 14.7 us with 256 threads, 10.5 with 512; 96 x 64: 13.3 and
+// 9.8). With more tiles than SMs two CTAs of 256 threads share an SM (512 threads: 2.5 % slower
+// at 4400 x 640).
+__host__ __device__ constexpr int stage_threads(int trt, bool wide = false) {
+  return wide ? 2 * STAGE_THREADS : (trt == TR ? STAGE_THREADS : STAGE_THREADS / 2);
+}
 template <typename R, int TRT>
-__host__ __device__ constexpr int stage_ctas() { return TRT == TR ? 2 : (rk_global<R, TRT>() ? 6 : 4); }
+__host__ __device__ constexpr int stage_ctas(bool wide = false) {
+  return wide ? 1 : (TRT == TR ? 2 : (rk_global<R, TRT>() ? 6 : 4));
+}
 
 // One tile per CTA; with TRT < TR (interior tiles only) CTA k takes rows (k % NH) * TRT ..
 // of tile k / NH, NH = TR / TRT.
-template <int H, bool GEN, typename SIN, typename R, int CM, int TRT = TR>
-__global__ void __launch_bounds__(stage_threads(TRT), (stage_ctas<R, TRT>()))
+template <int H, bool GEN, typename SIN, typename R, int CM, int TRT = TR, bool WIDE = false>
+__global__ void __launch_bounds__(stage_threads(TRT, WIDE), (stage_ctas<R, TRT>(WIDE)))
     stage_kernel(const StageArgs a, const int2* __restrict__ tiles, const __grid_constant__ CUtensorMap mState,
                  const __grid_constant__ CUtensorMap mQ, const __grid_constant__ CUtensorMap mU0,
                  const __grid_constant__ CUtensorMap mAcc, const __grid_constant__ CUtensorMap mB,
                  const __grid_constant__ CUtensorMap mTg) {
   static_assert(TRT == TR || !GEN, "general tiles run whole");
+  static_assert(GEN || !WIDE, "one point per thread: general tiles");
   constexpr int NH = TR / TRT;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar[2];
@@ -780,8 +930,8 @@ __global__ void __launch_bounds__(stage_threads(TRT), (stage_ctas<R, TRT>()))
   uint32_t phase = 0;
   const int2 t0 = tiles[blockIdx.x / NH];
   const int j0 = NH > 1 ? t0.y + (int)(blockIdx.x % NH) * TRT : t0.y;
-  stage_body<H, GEN, SIN, R, CM, stage_threads(TRT), TRT>(a, t0.x, j0, &mState, &mQ, &mU0, &mAcc, &mB, &mTg,
-                                                          smem_raw, bar, phase);
+  stage_body<H, GEN, SIN, R, CM, stage_threads(TRT, WIDE), TRT>(a, t0.x, j0, &mState, &mQ, &mU0, &mAcc, &mB, &mTg,
+                                                                smem_raw, bar, phase);
 }
 
 // Batched form: a persistent grid-stride loop over the tiles (i0, j0, instance) of many
@@ -789,7 +939,7 @@ __global__ void __launch_bounds__(stage_threads(TRT), (stage_ctas<R, TRT>()))
 // (the arguments are staged in shared memory per tile). With TRT < TR the table holds the
 // half tiles of the interior class (their own origins) and the maps their boxes.
 template <int H, bool GEN, typename SIN, typename R, int CM, int TRT = TR>
-__global__ void __launch_bounds__(stage_threads(TRT), TRT == TR ? 1 : (stage_ctas<R, TRT>()))
+__global__ void __launch_bounds__(stage_threads(TRT), GEN ? 2 : (TRT == TR ? 1 : (stage_ctas<R, TRT>())))
     stage_kernel_batch(const StageArgs* __restrict__ argv, const int4* __restrict__ tiles, int ntiles,
                        const CUtensorMap* __restrict__ mapv, int nmaps, int4 kmaps) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -816,25 +966,21 @@ __global__ void __launch_bounds__(stage_threads(TRT), TRT == TR ? 1 : (stage_cta
   }
 }
 
-template <int H, bool GEN, typename SIN, typename R, int TRT = TR>
+template <int H, bool GEN, typename SIN, typename R, int CM, int TRT, bool WIDE>
+static cudaError_t launch_stage_cm(const StageArgs& a, int ntiles, const int2* tiles, const StageMaps& m,
+                                   cudaStream_t s) {
+  const size_t sm = StageSmem<H, SIN, R, CM, TRT>::bytes(GEN);
+  stage_kernel<H, GEN, SIN, R, CM, TRT, WIDE><<<ntiles * (TR / TRT), stage_threads(TRT, WIDE), sm, s>>>(
+      a, tiles, *m.state, *m.star, *m.u0, *m.acc, *m.bt, *m.tg);
+  return cudaGetLastError();
+}
+template <int H, bool GEN, typename SIN, typename R, int TRT = TR, bool WIDE = false>
 static cudaError_t launch_stage_t(const StageArgs& a, int ntiles, const int2* tiles, const StageMaps& m,
                                   cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
-  const int grid = ntiles * (TR / TRT), nt = stage_threads(TRT);
-  if (a.learned == CM_LRN) {
-    const size_t sm = StageSmem<H, SIN, R, CM_LRN, TRT>::bytes(GEN);
-    stage_kernel<H, GEN, SIN, R, CM_LRN, TRT>
-        <<<grid, nt, sm, s>>>(a, tiles, *m.state, *m.star, *m.u0, *m.acc, *m.bt, *m.tg);
-  } else if (a.learned == CM_PRE) {
-    const size_t sm = StageSmem<H, SIN, R, CM_PRE, TRT>::bytes(GEN);
-    stage_kernel<H, GEN, SIN, R, CM_PRE, TRT>
-        <<<grid, nt, sm, s>>>(a, tiles, *m.state, *m.star, *m.u0, *m.acc, *m.bt, *m.tg);
-  } else {
-    const size_t sm = StageSmem<H, SIN, R, CM_FILT, TRT>::bytes(GEN);
-    stage_kernel<H, GEN, SIN, R, CM_FILT, TRT>
-        <<<grid, nt, sm, s>>>(a, tiles, *m.state, *m.star, *m.u0, *m.acc, *m.bt, *m.tg);
-  }
-  return cudaGetLastError();
+  if (a.learned == CM_LRN) return launch_stage_cm<H, GEN, SIN, R, CM_LRN, TRT, WIDE>(a, ntiles, tiles, m, s);
+  if (a.learned == CM_PRE) return launch_stage_cm<H, GEN, SIN, R, CM_PRE, TRT, WIDE>(a, ntiles, tiles, m, s);
+  return launch_stage_cm<H, GEN, SIN, R, CM_FILT, TRT, WIDE>(a, ntiles, tiles, m, s);
 }
 
 // The general tiles (few, heavy, one CTA per SM) run on a side stream next to the
@@ -852,13 +998,17 @@ static cudaError_t join(const SideStream& side, cudaStream_t s) {
   return cudaStreamWaitEvent(s, side.join, 0);
 }
 
+constexpr int STAGE_WIDE_TILES = 148;  // one general tile per SM
+
 template <typename SIN, typename R>
 static cudaError_t launch_stage_pair(const StageArgs& a, int ntiles_int, const int2* tiles_int, const StageMaps& mint,
                                      int ntiles_gen, const int2* tiles_gen, const StageMaps& mgen,
                                      const SideStream& side, cudaStream_t s, int int_rows) {
   cudaError_t e = fork(side, s);
   if (e != cudaSuccess) return e;
-  e = launch_stage_t<H_GEN, true, SIN, R>(a, ntiles_gen, tiles_gen, mgen, side.stream ? side.stream : s);
+  cudaStream_t gs = side.stream ? side.stream : s;
+  e = ntiles_gen <= STAGE_WIDE_TILES ? launch_stage_t<H_GEN, true, SIN, R, TR, true>(a, ntiles_gen, tiles_gen, mgen, gs)
+                                     : launch_stage_t<H_GEN, true, SIN, R>(a, ntiles_gen, tiles_gen, mgen, gs);
   if (e != cudaSuccess) return e;
   e = int_rows == TR / 2 ? launch_stage_t<H_INT, false, SIN, R, TR / 2>(a, ntiles_int, tiles_int, mint, s)
                         : launch_stage_t<H_INT, false, SIN, R>(a, ntiles_int, tiles_int, mint, s);
@@ -2542,17 +2692,27 @@ void sensor_boxes(bool gen, bool mixed, int* vw, int* vh, int* tw, int* th) {
   }
 }
 
-template <int H, bool GEN, typename SIN, typename R, int TRT = TR>
-static cudaError_t stage_attr() {
-  cudaError_t e = cudaFuncSetAttribute(stage_kernel<H, GEN, SIN, R, CM_FILT, TRT>,
+template <int H, bool GEN, typename SIN, typename R, int TRT, bool WIDE>
+static cudaError_t stage_attr_w() {
+  cudaError_t e = cudaFuncSetAttribute(stage_kernel<H, GEN, SIN, R, CM_FILT, TRT, WIDE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)StageSmem<H, SIN, R, CM_FILT, TRT>::bytes(GEN));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(stage_kernel<H, GEN, SIN, R, CM_PRE, TRT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  e = cudaFuncSetAttribute(stage_kernel<H, GEN, SIN, R, CM_PRE, TRT, WIDE>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)StageSmem<H, SIN, R, CM_PRE, TRT>::bytes(GEN));
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(stage_kernel<H, GEN, SIN, R, CM_LRN, TRT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(stage_kernel<H, GEN, SIN, R, CM_LRN, TRT, WIDE>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)StageSmem<H, SIN, R, CM_LRN, TRT>::bytes(GEN));
+}
+template <int H, bool GEN, typename SIN, typename R, int TRT = TR>
+static cudaError_t stage_attr() {
+  cudaError_t e = stage_attr_w<H, GEN, SIN, R, TRT, false>();
+  if constexpr (GEN) {
+    if (e == cudaSuccess) e = stage_attr_w<H, GEN, SIN, R, TRT, true>();
+  }
+  return e;
 }
 template <int HS, int HF, bool GEN, typename SIN, typename R>
 static cudaError_t sensor_attr() {
