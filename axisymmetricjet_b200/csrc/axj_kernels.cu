@@ -148,33 +148,14 @@ __device__ __forceinline__ R dot_c1(const S* p, int stride) {
   return s;
 }
 
-// Derivative stencil of table TAB with row code `row` (0..8; 9 = none) at p (pointer
-// to the point's own value), stride 1 along z or the row length along r. Interior
-// tiles (GEN = false) always use the centred row.
-template <typename R, int TAB, bool GEN, typename S>
-__device__ __forceinline__ R dst(int row, const S* p, int stride) {
-  if (!GEN || row == 4) {
-    if (TAB == 1) return dot_c1<R>(p, stride);
-    return dotc<R, TAB, 5>(4, p - 2 * stride, stride);
-  }
-  if (row >= 9) return R(0);
-  return dotc<R, TAB, 6>(row, p + sbp_w0(row) * stride, stride);
-}
-
-// dp/dz, dp/dr: the reference differentiates pvec = rhovec*Tvec, so every tap is a product.
-template <typename R, bool GEN, typename S>
-__device__ __forceinline__ R dst_p(int row, const S* rho, const S* T, int stride) {
-  int w0, n, rw;
-  if (!GEN || row == 4) { w0 = -2; n = 5; rw = 4; }
-  else if (row >= 9) return R(0);
-  else { w0 = sbp_w0(row); n = 6; rw = row; }
-  R s = tabv<R, 1>(rw, 0) * (R(rho[w0 * stride]) * R(T[w0 * stride]));
-#pragma unroll
-  for (int m = 1; m < 6; ++m) {
-    if (m >= n) continue;
-    if (rw == 4 && m == 2) continue;  // the centred row's exactly zero middle weight
-    s = s + tabv<R, 1>(rw, m) * (R(rho[(w0 + m) * stride]) * R(T[(w0 + m) * stride]));
-  }
+// dp/dz, dp/dr by the centred row: the reference differentiates pvec = rhovec*Tvec, so every
+// tap is a product (the exactly zero middle weight left out).
+template <typename R, typename S>
+__device__ __forceinline__ R dot_c1_p(const S* rho, const S* T, int stride) {
+  R s = tabv<R, 1>(4, 0) * (R(rho[-2 * stride]) * R(T[-2 * stride]));
+  s = s + tabv<R, 1>(4, 1) * (R(rho[-stride]) * R(T[-stride]));
+  s = s + tabv<R, 1>(4, 3) * (R(rho[stride]) * R(T[stride]));
+  s = s + tabv<R, 1>(4, 4) * (R(rho[2 * stride]) * R(T[2 * stride]));
   return s;
 }
 
@@ -227,7 +208,7 @@ __device__ __forceinline__ R dst6(const Row6<R>& q, const S* p, int stride) {
 template <typename R, bool C, typename S>
 __device__ __forceinline__ R dst6_p(const Row6<R>& q, const S* rho, const S* T, int stride) {
   if constexpr (C) {
-    return dst_p<R, false>(4, rho, T, stride);
+    return dot_c1_p<R>(rho, T, stride);
   } else {
     const S *a = rho + q.w0 * stride, *b = T + q.w0 * stride;
     R s = q.a[0] * (R(a[0]) * R(b[0]));
@@ -235,16 +216,6 @@ __device__ __forceinline__ R dst6_p(const Row6<R>& q, const S* rho, const S* T, 
     for (int m = 1; m < 5; ++m) s = s + q.a[m] * (R(a[m * stride]) * R(b[m * stride]));
     return s + q.a[5] * (R(rho[q.o5 * stride]) * R(T[q.o5 * stride]));
   }
-}
-
-// 9-point fourth difference cC9 centred at p (stride in elements), left to right.
-template <typename R, typename S>
-__device__ __forceinline__ R c9dot(const S* p, int stride) {
-  const R* c = std::is_same<R, float>::value ? reinterpret_cast<const R*>(cC9f) : reinterpret_cast<const R*>(cC9);
-  R s = c[0] * R(p[-4 * stride]);
-#pragma unroll
-  for (int m = 1; m < 9; ++m) s = s + c[m] * R(p[(m - 4) * stride]);
-  return s;
 }
 
 // axis_conditions (ModAxis.f90:14-16): f(1) = -DOT_PRODUCT(SBP1(0,1:5), f(2:6)) / SBP1(0,0),
@@ -1257,15 +1228,18 @@ struct SensSmem {
   // T [SR][SZ] (TMA); S and dil [SR][SZ]; general tiles: descriptors [VR][VZ]. V and T
   // are in the stage-input type, the rest in the stencil type. Once phase 2 has formed the
   // strain rates the V boxes are spent: f_sw [TR][TZ] then lives in the V_r box (interior
-  // tiles) or the V_z box (general tiles), and the general tiles' second derivatives on the
-  // arms ([TR][DZ] + [DR][TZ]) in the V_r box. rho is read from the stage input.
+  // tiles) or the V_z box's end (general tiles), and the general tiles' second derivatives of
+  // the three fields on the arms ([TR][DZ] + [DR][TZ] each) from the V_r box on. rho is read
+  // from the stage input.
   static constexpr size_t oVr = 0;
   static constexpr size_t oVz = align128(sizeof(SIN) * NV);
   static constexpr size_t oT = align128(oVz + sizeof(SIN) * NV);
   static constexpr size_t oS = align128(oT + sizeof(SIN) * NS);
   static constexpr size_t oD = align128(oS + sizeof(R) * NS);
-  static_assert(sizeof(R) * (TR * DZ + DR * TZ) <= sizeof(SIN) * NV && sizeof(R) * TR * TZ <= sizeof(SIN) * NV,
-                "the arms and f_sw fit in a spent V box");
+  static constexpr int NARM = TR * DZ + DR * TZ;
+  static constexpr size_t oFswGen = (oVz + sizeof(SIN) * NV - sizeof(R) * TR * TZ) / 16 * 16;
+  static_assert(HF == 2 || (sizeof(R) * 3 * NARM <= oFswGen && sizeof(R) * TR * TZ <= sizeof(SIN) * NV),
+                "the arms and f_sw fit in the spent V boxes");
   static constexpr size_t oDesc = align128(oD + sizeof(R) * NS);
   // metrics of the S region: dxidz on its columns [SZ], detadr and 1/r on its rows
   // [2][SR]; deltaz, deltar on the tile [TZ] + [TR]
@@ -1273,12 +1247,19 @@ struct SensSmem {
     return align128(oDesc + (gen ? sizeof(uint32_t) * NV : 0));
   }
   static constexpr int NMET = SZ + 2 * SR + TZ + TR;
-  __host__ __device__ static constexpr size_t bytes(bool gen) { return align128(oMet(gen) + sizeof(double) * NMET); }
+  // general tiles: the six-tap stencil rows
+  __host__ __device__ static constexpr size_t oRow(bool gen) { return align128(oMet(gen) + sizeof(double) * NMET); }
+  __host__ __device__ static constexpr size_t bytes(bool gen) {
+    return align128(oRow(gen) + (gen ? sizeof(R) * ROW6_ROWS * 12 : 0));
+  }
   static constexpr uint32_t tx_bytes = sizeof(SIN) * (2 * NV + NS);
 };
 
 // Threads of a sensor tile CTA: general tiles 512, one point per thread in the stencil
-// phases (two CTAs per SM at 105 KB of shared memory and 64 registers); interior tiles
+// phases (two CTAs per SM at 106 KB of shared memory and 64 registers). A general tile's latency
+// bounds them; with the loads grouped, one branch per warp and direction, the three fields'
+// arms in one pass and the band's own rows only, measured on a B200: 96 x 64 12.2 -> 8.8 us,
+// 787 x 203 14.1 -> 10.4, 4400 x 640 22.4 -> 15.7, a batch of 12 jets (mixed) 46.8 -> 31.4; interior tiles
 // 128, a 2 x 2 block of points per thread (five CTAs per SM at 44 KB).
 __host__ __device__ constexpr int sens_threads(bool gen) { return gen ? 512 : 128; }
 
@@ -1316,15 +1297,6 @@ __device__ __forceinline__ R c1_of(R xm2, R xm1, R xp1, R xp2) {
   s = s + tabv<R, 1>(4, 4) * xp2;
   return s;
 }
-// The 9-point fourth difference cC9 on x[0..8], left to right (c9dot's order).
-template <typename R>
-__device__ __forceinline__ R c9_of(const R* x) {
-  const R* c = std::is_same<R, float>::value ? reinterpret_cast<const R*>(cC9f) : reinterpret_cast<const R*>(cC9);
-  R s = c[0] * x[0];
-#pragma unroll
-  for (int m = 1; m < 9; ++m) s = s + c[m] * x[m];
-  return s;
-}
 template <>
 __device__ __forceinline__ float sqrt_t<float>(float x) { return sqrtf(x); }
 
@@ -1342,10 +1314,10 @@ __device__ __forceinline__ bool sensor_body(const SensorArgs& a, int i0, int j0,
   SIN* sT = reinterpret_cast<SIN*>(smem_raw + SM::oT);     // [SR][SZ]
   R* sS = reinterpret_cast<R*>(smem_raw + SM::oS);         // [SR][SZ]
   R* sD = reinterpret_cast<R*>(smem_raw + SM::oD);         // [SR][SZ]
-  R* sd2z = reinterpret_cast<R*>(smem_raw + SM::oVr);      // [TR][DZ] (general tiles, phase 3)
-  R* sd2r = sd2z + TR * DZ;                                 // [DR][TZ] (general tiles, phase 3)
+  R* sArm = reinterpret_cast<R*>(smem_raw + SM::oVr);      // [3][TR][DZ + DR][TZ] (general tiles, phase 3)
+  R* sRow = reinterpret_cast<R*>(smem_raw + SM::oRow(GEN));  // [ROW6_ROWS][12] (general tiles)
   // f_sw [TR][TZ] in a spent V box (after phase 2): V_z (general tiles) or V_r (interior)
-  R* sFsw = reinterpret_cast<R*>(smem_raw + (GEN ? SM::oVz : SM::oVr));
+  R* sFsw = reinterpret_cast<R*>(smem_raw + (GEN ? SM::oFswGen : SM::oVr));
   const SIN* rho0 = std::is_same<SIN, float>::value ? reinterpret_cast<const SIN*>(a.Uf)
                                                      : reinterpret_cast<const SIN*>(a.U);  // rho plane
   uint32_t* sDesc = reinterpret_cast<uint32_t*>(smem_raw + SM::oDesc);
@@ -1365,7 +1337,6 @@ __device__ __forceinline__ bool sensor_body(const SensorArgs& a, int i0, int j0,
     j0 &= 0xFFFFFF;
   }
   auto inside = [&](int i, int j) { return i >= 0 && i < Nz && j >= 0 && j < Nr; };
-  auto vdesc = [&](int vidx) -> uint32_t { return GEN ? sDesc[vidx] : make_desc(4, 4, false, 0); };
 
   // ---- phase 1: V_r, V_z on the V region, T on the S region and rho on the tile by
   // TMA (zero outside the block), descriptors by plain loads meanwhile. The barrier is
@@ -1392,13 +1363,6 @@ __device__ __forceinline__ bool sensor_body(const SensorArgs& a, int i0, int j0,
       rho_pf[w][1] = v.y;
     }
   }
-  if (GEN) {
-    for (int idx = tid; idx < NV; idx += NT) {
-      const int vr = idx / VZ, vz = idx - vr * VZ;
-      const int i = i0 - HVZ + vz, j = j0 - HV + vr;
-      sDesc[idx] = inside(i, j) ? __ldg(a.desc + (long long)j * g.P + i) : make_desc(ROW_NONE, ROW_NONE, false, 0);
-    }
-  }
   // metrics and coordinates of the region (clamped indices: values outside the grid are
   // never used)
   for (int k = tid; k < SM::NMET; k += NT) {
@@ -1414,6 +1378,28 @@ __device__ __forceinline__ bool sensor_body(const SensorArgs& a, int i0, int j0,
       v = __ldg(a.dr + min(j0 + (k - SZ - 2 * SM::SR - TZ), Nr - 1));
     }
     sMz[k] = v;
+  }
+  SIN rho_g = SIN(0);  // general tiles: rho of the thread's tile point
+  if constexpr (GEN) {
+    // descriptors of the V region and rho, all of a thread's loads in flight
+    constexpr int ND = (NV + NT - 1) / NT;
+    uint32_t dv[ND];
+#pragma unroll
+    for (int q = 0; q < ND; ++q) {
+      const int idx = tid + q * NT;
+      const int vr = idx / VZ, vz = idx - vr * VZ;
+      const int i = i0 - HVZ + vz, j = j0 - HV + vr;
+      dv[q] = idx < NV && inside(i, j) ? __ldg(a.desc + (long long)j * g.P + i)
+                                       : make_desc(ROW_NONE, ROW_NONE, false, 0);
+    }
+    {
+      const int i = i0 + (tid & (TZ - 1)), j = j0 + tid / TZ;
+      if (inside(i, j)) rho_g = __ldg(rho0 + (long long)j * g.P + i);
+    }
+    row6_fill(sRow, tid, NT);
+#pragma unroll
+    for (int q = 0; q < ND; ++q)
+      if (tid + q * NT < NV) sDesc[tid + q * NT] = dv[q];
   }
   if (!__syncthreads_and(mbar_wait_bounded(&bar, phase & 1u))) {
     if (tid == 0) atomicOr(a.flags, 4);
@@ -1557,55 +1543,71 @@ __device__ __forceinline__ bool sensor_body(const SensorArgs& a, int i0, int j0,
       }
     }
   } else {
+    // general tiles: the rows the band's own rows reach; a warp branches once per direction,
+    // between the centred row and the six-tap form of any row
+    const int rows = nrow + 2 * HS;
 #pragma unroll
-  for (int u = 0; u < NSIT; ++u) {
-    const int idx = tid + u * NT;
-    if (idx >= NS) break;
-    const int sr = idx / SZ, sz = idx - sr * SZ;
-    const bool zarm = sr >= HS && sr < HS + TR && sz >= HSZ - HS && sz < HSZ + TZ + HS;
-    const bool rarm = sz >= HSZ && sz < HSZ + TZ;
-    R S = R(0), dil = R(0);
-    const int i = i0 - HSZ + sz, j = j0 - HS + sr;
-    if ((zarm || rarm) && (!GEN || inside(i, j))) {
-      const int vidx = (sr + HV - HS) * VZ + (sz + HVZ - HSZ);
-      const uint32_t dsc = vdesc(vidx);
-      const int zr = desc_blank(dsc) ? (int)ROW_NONE : desc_zrow(dsc);
-      const int rw = desc_blank(dsc) ? (int)ROW_NONE : desc_rrow(dsc);
-      const R xz = R(sMz[sz]), er = R(sMr[sr]);
-      const R dVrdz = dst<R, 1, GEN>(zr, sVr + vidx, 1) * xz;
-      const R dVzdz = dst<R, 1, GEN>(zr, sVz + vidx, 1) * xz;
-      const R dVrdr = dst<R, 1, GEN>(rw, sVr + vidx, VZ) * er;
-      const R dVzdr = dst<R, 1, GEN>(rw, sVz + vidx, VZ) * er;
-      const R vr = R(sVr[vidx]);
-      // V_r / r as V_r * (1/r) (the reference divides; the two differ by rounding)
-      const R vr_r = vr * R(sIr[sr]);
-      if (j == 0) dil = R(2.0) * dVrdr + dVzdz;
-      else dil = dVrdr + vr_r + dVzdz;
-      const R S11 = dVrdr - R(1.0 / 3.0) * dil;
-      const R S13 = R(0.5) * (dVrdz + dVzdr);
-      const R S33 = dVzdz - R(1.0 / 3.0) * dil;
-      const R S22 = (j == 0) ? dVrdr - R(1.0 / 3.0) * dil : vr_r - R(1.0 / 3.0) * dil;
-      S = sqrt_t<R>(S11 * S11 + S13 * S13 + S22 * S22 + S13 * S13 + S33 * S33);
-      if (zarm && rarm) {
-        const R vort = fabs(dVrdz - dVzdr);
-        const R Hm = (R(-1.0) * dil < R(0)) ? R(0) : R(1);
-        const R eps = R((double)1e-15f);  // single-precision literal of the reference (:202)
-        // kept in registers: the V_z box that holds f_sw is still being read
-        fkg[u] = Hm * (dil * dil) / (dil * dil + vort * vort + eps);
-        fig[u] = (sr - HS) * TZ + (sz - HSZ);
+    for (int u = 0; u < NSIT; ++u) {
+      const int idx = tid + u * NT;
+      const int sr = idx / SZ, sz = idx - sr * SZ;
+      const bool zarm = sr >= HS && sr < HS + nrow && sz >= HSZ - HS && sz < HSZ + TZ + HS;
+      const bool rarm = sr < rows && sz >= HSZ && sz < HSZ + TZ;
+      const int i = i0 - HSZ + sz, j = j0 - HS + sr;
+      const bool act = (zarm || rarm) && inside(i, j);
+      R S = R(0), dil = R(0);
+      if (__any_sync(0xffffffffu, act)) {
+        const int vidx = act ? (sr + HV - HS) * VZ + (sz + HVZ - HSZ) : HV * VZ + HVZ;
+        const int sq = act ? sr : 0, zq = act ? sz : 0;
+        const uint32_t dsc = act ? sDesc[vidx] : make_desc(4, 4, false, 0);
+        const int zr = desc_blank(dsc) ? (int)ROW_NONE : desc_zrow(dsc);
+        const int rw = desc_blank(dsc) ? (int)ROW_NONE : desc_rrow(dsc);
+        R gzr, gzz, grr, grz;
+        auto pair_d1 = [&](auto centred, int row, int stride, R& gr, R& gz) {
+          constexpr bool C = decltype(centred)::value;
+          Row6<R> q;
+          if constexpr (!C) q = row6(sRow, row);
+          gr = dst6<R, C, 1>(q, sVr + vidx, stride);
+          gz = dst6<R, C, 1>(q, sVz + vidx, stride);
+          if (!C && row >= 9) gr = gz = R(0);
+        };
+        if (__all_sync(0xffffffffu, zr == 4)) pair_d1(std::true_type{}, 4, 1, gzr, gzz);
+        else pair_d1(std::false_type{}, zr, 1, gzr, gzz);
+        if (__all_sync(0xffffffffu, rw == 4)) pair_d1(std::true_type{}, 4, VZ, grr, grz);
+        else pair_d1(std::false_type{}, rw, VZ, grr, grz);
+        const R xz = R(sMz[zq]), er = R(sMr[sq]);
+        const R dVrdz = gzr * xz, dVzdz = gzz * xz, dVrdr = grr * er, dVzdr = grz * er;
+        // V_r / r as V_r * (1/r) (the reference divides; the two differ by rounding)
+        const R vr_r = R(sVr[vidx]) * R(sIr[sq]);
+        if (j == 0) dil = R(2.0) * dVrdr + dVzdz;
+        else dil = dVrdr + vr_r + dVzdz;
+        const R S11 = dVrdr - R(1.0 / 3.0) * dil;
+        const R S13 = R(0.5) * (dVrdz + dVzdr);
+        const R S33 = dVzdz - R(1.0 / 3.0) * dil;
+        const R S22 = (j == 0) ? dVrdr - R(1.0 / 3.0) * dil : vr_r - R(1.0 / 3.0) * dil;
+        S = sqrt_t<R>(S11 * S11 + S13 * S13 + S22 * S22 + S13 * S13 + S33 * S33);
+        if (act && zarm && rarm) {
+          const R vort = fabs(dVrdz - dVzdr);
+          const R Hm = (R(-1.0) * dil < R(0)) ? R(0) : R(1);
+          const R eps = R((double)1e-15f);  // single-precision literal of the reference (:202)
+          // kept in registers: the V_z box that holds f_sw is still being read
+          fkg[u] = Hm * (dil * dil) / (dil * dil + vort * vort + eps);
+          fig[u] = (sr - HS) * TZ + (sz - HSZ);
+        }
+        if (!act) S = dil = R(0);
+      }
+      if (idx < NS) {
+        sS[idx] = S;
+        sD[idx] = dil;
       }
     }
-    sS[idx] = S;
-    sD[idx] = dil;
-  }
   }
   __syncthreads();
   if constexpr (GEN) {
-    // every thread is done with the V boxes: f_sw into the V_z box
+    // every thread is done with the V boxes: f_sw to the V_z box's end
 #pragma unroll
     for (int u = 0; u < NSIT; ++u)
       if (fig[u] >= 0) sFsw[fig[u]] = fkg[u];
-    __syncthreads();
+    // (read after the arms' barrier; the arms lie elsewhere in the spent boxes)
   }
   if constexpr (!GEN) {
     // every thread is done with the V boxes: f_sw into the V_r box
@@ -1618,23 +1620,17 @@ __device__ __forceinline__ bool sensor_body(const SensorArgs& a, int i0, int j0,
     __syncthreads();
   }
 
-  // ---- phases 3-4 per field: fourth derivatives at the tile points (kept in registers:
-  // PPT points per thread, 4 in interior tiles, 1 in general tiles, the general tiles'
-  // arms in the spent V_r box). Interior tiles: SBP2 of SBP2 with the centred row both times is
-  // the 9-point row cC9 = c * c (c the centred SBP2 row), applied to S, T, the dilatation
-  // directly (one rounding per product instead of two stencil passes: the difference is
-  // rounding only). General tiles: second derivatives on the arms with each arm point's
-  // row, then the tile point's row.
-  constexpr int PPT = (TZ * TR) / NT;
-  // point q of a thread: a warp owns PPT consecutive rows of the tile, so a thread's
-  // points are vertically adjacent and share most taps of their r stencils (loaded once)
-  auto ppoint = [](int t, int q) { return (t >> 5) * (TZ * PPT) + q * TZ + (t & 31); };
-  R d4z[3][PPT], d4r[3][PPT];
+  // ---- phases 3-4: fourth derivatives at the tile points. Interior tiles: SBP2 of SBP2 with
+  // the centred row both times is the 9-point row cC9 = c * c (c the centred SBP2 row), applied
+  // to S, T, the dilatation directly (one rounding per product instead of two stencil passes:
+  // the difference is rounding only). General tiles: second derivatives of the three fields on
+  // the arms with each arm point's row (in the spent V boxes), then the tile point's row, one
+  // point per thread.
   if constexpr (!GEN) {
     // 2 x 2 blocks of points (rows r, r + 1 and columns c, c + 1; r, c even), every window
     // in pair loads: along z each block row's five pairs (columns c - 4 .. c + 5) serve its
     // two points, along r each of the ten rows r - 4 .. r + 5 serves the block rows it
-    // reaches. Every point's sum keeps c9dot's order (taps left to right). The quantities
+    // reaches. Every point's sum takes its taps left to right. The quantities
     // of a field leave as soon as its sums are complete.
     static_assert(NT * 4 == TZ * TR, "one 2 x 2 block of points per thread");
     const int r = 2 * (tid / (TZ / 2)), c = 2 * (tid - (tid / (TZ / 2)) * (TZ / 2));
@@ -1748,67 +1744,78 @@ __device__ __forceinline__ bool sensor_body(const SensorArgs& a, int i0, int j0,
     for (int w = 0; w < 2; ++w) st_pair(a.Q + 2 * g.plane + o + w * g.P, out[w][0], out[w][1]);
     return true;
   } else {
+    static_assert(NT == TZ * TR, "one tile point per thread");
+    constexpr int NARM = SM::NARM;
+    const int nz = nrow * DZ, na = nz + (nrow + 2 * HF) * TZ;
+    // arm points of both directions in one list: one code path with the direction's stride
 #pragma unroll
-  for (int f = 0; f < 3; ++f) {
-    for (int idx = tid; idx < TR * DZ + DR * TZ; idx += NT) {
-      if (idx < TR * DZ) {
-        const int r = idx / DZ, c = idx - r * DZ;  // point (i0 - HF + c, j0 + r)
-        const int i = i0 - HF + c, j = j0 + r;
-        R v = R(0);
-        if (!GEN || inside(i, j)) {
-          const int sidx = (HS + r) * SZ + (HSZ - HF + c);
-          const uint32_t dsc = vdesc((HV + r) * VZ + (HVZ - HF + c));
-          const int zr = desc_blank(dsc) ? (int)ROW_NONE : desc_zrow(dsc);
-          v = f == 1 ? dst<R, 2, GEN>(zr, sT + sidx, 1) : dst<R, 2, GEN>(zr, (f == 0 ? sS : sD) + sidx, 1);
-        }
-        sd2z[idx] = v;
-      } else {
-        const int k = idx - TR * DZ;
-        const int r = k / TZ, c = k - r * TZ;      // point (i0 + c, j0 - HF + r)
-        const int i = i0 + c, j = j0 - HF + r;
-        R v = R(0);
-        if (!GEN || inside(i, j)) {
-          const int sidx = (HS - HF + r) * SZ + (HSZ + c);
-          const uint32_t dsc = vdesc((HV - HF + r) * VZ + (HVZ + c));
-          const int rw = desc_blank(dsc) ? (int)ROW_NONE : desc_rrow(dsc);
-          v = f == 1 ? dst<R, 2, GEN>(rw, sT + sidx, SZ) : dst<R, 2, GEN>(rw, (f == 0 ? sS : sD) + sidx, SZ);
-        }
-        sd2r[k] = v;
+    for (int u = 0; u < (NARM + NT - 1) / NT; ++u) {
+      const int idx = tid + u * NT;
+      if (u * NT >= na) break;  // uniform
+      const bool za = idx < nz;
+      const int k = za ? idx : idx - nz;
+      const int r = za ? k / DZ : k / TZ, c = za ? k - r * DZ : k - r * TZ;
+      // z arm: point (i0 - HF + c, j0 + r); r arm: (i0 + c, j0 - HF + r)
+      const int i = za ? i0 - HF + c : i0 + c, j = za ? j0 + r : j0 - HF + r;
+      const bool act = idx < na && inside(i, j);
+      const int sidx = !act ? HS * SZ + HSZ : (za ? (HS + r) * SZ + (HSZ - HF + c) : (HS - HF + r) * SZ + (HSZ + c));
+      const int stride = za ? 1 : SZ;
+      int row = 4;
+      if (act) {
+        const uint32_t dsc = sDesc[za ? (HV + r) * VZ + (HVZ - HF + c) : (HV - HF + r) * VZ + (HVZ + c)];
+        row = desc_blank(dsc) ? (int)ROW_NONE : (za ? desc_zrow(dsc) : desc_rrow(dsc));
+      }
+      R v[3];
+      auto second = [&](auto centred) {
+        constexpr bool C = decltype(centred)::value;
+        Row6<R> q;
+        if constexpr (!C) q = row6(sRow, row);
+        v[0] = dst6<R, C, 2>(q, sS + sidx, stride);
+        v[1] = dst6<R, C, 2>(q, sT + sidx, stride);
+        v[2] = dst6<R, C, 2>(q, sD + sidx, stride);
+      };
+      if (__all_sync(0xffffffffu, row == 4)) second(std::true_type{});
+      else second(std::false_type{});
+      if (!act || row >= 9) v[0] = v[1] = v[2] = R(0);
+      if (idx < na) {
+        R* arm = sArm + (za ? k : TR * DZ + k);
+#pragma unroll
+        for (int f = 0; f < 3; ++f) arm[f * NARM] = v[f];
       }
     }
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-      const int pidx = ppoint(tid, q);
-      const int r = pidx / TZ, c = pidx - r * TZ;
-      const uint32_t dsc = vdesc((HV + r) * VZ + (HVZ + c));
-      const int zr = desc_blank(dsc) ? (int)ROW_NONE : desc_zrow(dsc);
-      const int rw = desc_blank(dsc) ? (int)ROW_NONE : desc_rrow(dsc);
-      d4z[f][q] = dst<R, 2, GEN>(zr, sd2z + r * DZ + HF + c, 1);
-      d4r[f][q] = dst<R, 2, GEN>(rw, sd2r + (HF + r) * TZ + c, TZ);
-    }
-    __syncthreads();
-  }
-  }
-
-  // ---- quantities to be filtered (ComputeTobeFilteredQuantities :204-215); the interior
-  // tiles returned above
-  if constexpr (GEN) {
-#pragma unroll
-  for (int q = 0; q < PPT; ++q) {
-    const int pidx = ppoint(tid, q);
-    const int r = pidx / TZ, c = pidx - r * TZ;
+    // ---- quantities to be filtered (ComputeTobeFilteredQuantities :204-215)
+    const int r = tid / TZ, c = tid - r * TZ;
+    if (r >= nrow) return true;  // whole warps
     const int i = i0 + c, j = j0 + r;
-    if (!inside(i, j) || r >= nrow) continue;
+    const bool in = inside(i, j);
+    const uint32_t dsc = in ? sDesc[(HV + r) * VZ + (HVZ + c)] : make_desc(4, 4, false, 0);
+    const int zr = desc_blank(dsc) ? (int)ROW_NONE : desc_zrow(dsc);
+    const int rw = desc_blank(dsc) ? (int)ROW_NONE : desc_rrow(dsc);
+    R dz4[3], dr4[3];
+    auto fourth = [&](auto centred, int row, const R* base, int stride, R (&d)[3]) {
+      constexpr bool C = decltype(centred)::value;
+      Row6<R> q;
+      if constexpr (!C) q = row6(sRow, row);
+#pragma unroll
+      for (int f = 0; f < 3; ++f) {
+        d[f] = dst6<R, C, 2>(q, base + f * NARM, stride);
+        if (!C && row >= 9) d[f] = R(0);
+      }
+    };
+    if (__all_sync(0xffffffffu, zr == 4)) fourth(std::true_type{}, 4, sArm + r * DZ + HF + c, 1, dz4);
+    else fourth(std::false_type{}, zr, sArm + r * DZ + HF + c, 1, dz4);
+    if (__all_sync(0xffffffffu, rw == 4)) fourth(std::true_type{}, 4, sArm + TR * DZ + (HF + r) * TZ + c, TZ, dr4);
+    else fourth(std::false_type{}, rw, sArm + TR * DZ + (HF + r) * TZ + c, TZ, dr4);
+    if (!in) return true;
     const long long o = (long long)j * g.P + i;
     const R dz = R(sDzv[c]), dr = R(sDrv[r]);
-    const R rho = R(rho0[o]);
+    const R rho = R(rho_g);
     const R T = R(sT[(HS + r) * SZ + HSZ + c]);
     const R fsw = sFsw[r * TZ + c];
-    a.Q[o] = double(rho * fabs((d4z[0][q] * (dz * dz) + d4r[0][q] * (dr * dr))));
-    a.Q[g.plane + o] = double(rho * fsw * fabs((d4z[2][q] * (dz * dz) + d4r[2][q] * (dr * dr))));
-    a.Q[2 * g.plane + o] = double(rho / (R(a.c.gam) * sqrt_t<R>(T)) * fabs((d4z[1][q] * dz + d4r[1][q] * dr)));
-  }
+    a.Q[o] = double(rho * fabs((dz4[0] * (dz * dz) + dr4[0] * (dr * dr))));
+    a.Q[g.plane + o] = double(rho * fsw * fabs((dz4[2] * (dz * dz) + dr4[2] * (dr * dr))));
+    a.Q[2 * g.plane + o] = double(rho / (R(a.c.gam) * sqrt_t<R>(T)) * fabs((dz4[1] * dz + dr4[1] * dr)));
   }
   return true;
 }
