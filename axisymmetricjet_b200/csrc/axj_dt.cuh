@@ -17,7 +17,7 @@
 // Measured at 4400 x 640 on a B200: the allocation-free kernel 51.4 -> 19.7 us (a call 57.4 ->
 // 22.6 us), the handle's 35.7 -> 23.0 us; what remains is issue (62 % of the active cycles) and
 // the launch's head and tail. Unscreened at 512 x 128 (one strip row per warp, a grid sized to
-// the points): 6.8 -> 5.5 us, where the screened form took 12.4.
+// the points): 6.8 -> 5.5 us.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -31,10 +31,12 @@ namespace axj {
 // than a block waste at most part of a strip.
 constexpr int DT_K = 4;
 constexpr int DT_WARPS = DT_THREADS / 32;
-// Grids up to this many points are scanned in FP64 throughout, one point per thread: with
-// under two points for every resident thread the screen's extra barrier and second pass cost
-// more than the FP64 work they save.
-constexpr long long DT_FULL = 148ll * 8 * DT_THREADS;
+// Grids up to this many points are scanned in FP64 throughout, one point per thread: the
+// screen's second pass then costs more than the FP64 work it saves. Measured (full / screened),
+// the handle's kernel: 38,400 points 5.2 / 6.1 us, 180,000 9.5 / 6.3, 400,000 13.2 / 8.1, 1.28 M
+// 34 / 14.6; a call of the allocation-free entry point: 65,536 points 11.6 / 11.6 us, 180,000
+// 12.3 / 10.4, 400,000 16.4 / 10.9, 2.8 M 63.6 / 22.5.
+constexpr long long DT_FULL = 98304;
 __host__ __device__ constexpr bool dt_screened(long long npts) { return npts > DT_FULL; }
 __host__ __device__ constexpr int dt_rows(bool screen) { return screen ? DT_K : 1; }
 // Strips of a grid, and the blocks that take one strip per warp.

@@ -70,9 +70,9 @@ def _noalloc(pv, dxidz, detadr, params, ib=None, stale=1.0, pad=5):
     return float(dt.item())
 
 
-# below, at and above the size from which the scan is screened (303,104 points), rows shorter
+# below, at and above the size from which the scan is screened (98,304 points), rows shorter
 # and longer than a block, ragged last chunks
-SIZES = [(1, 1), (12, 13), (255, 9), (4400, 7), (4736, 64), (4737, 64), (13, 23317), (257, 1283), (4400, 160),
+SIZES = [(1, 1), (12, 13), (255, 9), (4400, 7), (1536, 64), (1537, 64), (4737, 64), (13, 23317), (257, 1283), (4400, 160),
          (1, 2097153), (33, 270000)]  # the last two: more strips than the scratch has places
 
 
