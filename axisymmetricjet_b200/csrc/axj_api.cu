@@ -8,6 +8,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -29,6 +30,48 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
+}  // namespace
+
+// Page-locked places of 64 bytes for the handles' step scalars: a page-locked allocation takes
+// about 2 ms, half of a small handle's creation, so handles share pages of 64 places. A page is
+// allocated when none has a free place and given back when its last place is.
+namespace {
+struct PinPool {
+  static constexpr int kPlaces = 64, kDoubles = 8;
+  struct Page {
+    double* base;
+    uint64_t used;
+  };
+  std::mutex lock;
+  std::vector<Page> pages;
+  double* get() {
+    std::lock_guard<std::mutex> g(lock);
+    for (Page& p : pages)
+      if (~p.used) {
+        const int k = __builtin_ctzll(~p.used);
+        p.used |= 1ull << k;
+        return p.base + k * kDoubles;
+      }
+    void* m = nullptr;
+    if (cudaHostAlloc(&m, kPlaces * kDoubles * sizeof(double), cudaHostAllocPortable) != cudaSuccess) return nullptr;
+    pages.push_back(Page{static_cast<double*>(m), 1ull});
+    return pages.back().base;
+  }
+  void put(double* q) {
+    std::lock_guard<std::mutex> g(lock);
+    for (size_t k = 0; k < pages.size(); ++k) {
+      Page& p = pages[k];
+      if (q < p.base || q >= p.base + kPlaces * kDoubles) continue;
+      p.used &= ~(1ull << ((q - p.base) / kDoubles));
+      if (!p.used) {
+        cudaFreeHost(p.base);
+        pages.erase(pages.begin() + (long)k);
+      }
+      return;
+    }
+  }
+};
+PinPool g_pins;
 }  // namespace
 
 struct axj_handle {
@@ -1345,7 +1388,7 @@ void axj_destroy(axj_handle* h) {
     if (h->graph_rk4[k]) cudaGraphDestroy(h->graph_rk4[k]);
   }
   for (void* p : h->allocs) cudaFree(p);
-  if (h->pin) cudaFreeHost(h->pin);
+  if (h->pin) g_pins.put(h->pin);
   if (h->ds_feat) cudaFree(h->ds_feat);
   if (h->ds_targ) cudaFree(h->ds_targ);
   if (h->side.stream) cudaStreamSynchronize(h->side.stream);
@@ -1564,8 +1607,7 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
     h->staleT = h->dt + 2;
     h->flags = reinterpret_cast<int*>(h->dt + 3);
   }
-  if (rc == AXJ_OK && cudaHostAlloc(reinterpret_cast<void**>(&h->pin), 6 * sizeof(double), cudaHostAllocDefault) != cudaSuccess)
-    rc = fail(h, AXJ_ERR_NOMEM, "cudaHostAlloc of the step scalars failed");
+  if (rc == AXJ_OK && !(h->pin = g_pins.get())) rc = fail(h, AXJ_ERR_NOMEM, "page-locked memory for the step scalars");
   h->harm = dalloc<double>(h, 5, &rc);
 
   h->counter = dalloc<unsigned int>(h, 2, &rc);
