@@ -121,10 +121,38 @@ __device__ __forceinline__ float tanh_fast(float x) {
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float gelu_fast(float x) {
-  const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-  const float hx = 0.5f * x;
-  return fmaf(hx, tanh_fast(u), hx);
+// Two FP32 values in one 64-bit register pair, for the packed FP32 instructions (each half
+// rounded as the scalar instruction rounds it; one issue slot for two operations).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float x, float y) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+  return v;
+}
+__device__ __forceinline__ void unpk2(f32x2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// The tanh-form GELU of two values: 0.5 x (1 + tanh(x (k + 0.044715 k x^2))), k = sqrt(2/pi).
+__device__ __forceinline__ f32x2 gelu_fast2(f32x2 x) {
+  constexpr float k = 0.7978845608028654f;
+  const f32x2 u = mul2(x, fma2(mul2(x, x), pk2(0.044715f * k, 0.044715f * k), pk2(k, k)));
+  const f32x2 hx = mul2(x, pk2(0.5f, 0.5f));
+  float u0, u1;
+  unpk2(u, u0, u1);
+  return fma2(hx, pk2(tanh_fast(u0), tanh_fast(u1)), hx);
 }
 __device__ __forceinline__ float gelu_f(float x) {
   const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
@@ -264,9 +292,12 @@ cudaError_t launch_features(const FeatArgs& a, cudaStream_t s) {
 // layer-1 inputs and then (after the layer-1 MMAs completed) the layer-2 inputs, all
 // in the no-swizzle K-major layout with the K chunks outermost (chunk c of 8 K values
 // at c * rows * 16, row group g at g * 128, row r of the group at r * 16); the
-// normalised channel box 4 x 8 x 36 in BF16; biases and layer 3 in FP32. The next
-// tile's channel box is loaded into registers while this tile's MMAs run. About 54 KB
-// per CTA: 4 CTAs (16 warps, 256 TMEM columns) per SM.
+// normalised channel box 4 x 8 x 36 in BF16, twice (the second copy one value on); biases and
+// layer 3 in FP32. The next tile's channel box is loaded into registers while this tile's MMAs
+// run. About 57 KB per CTA: 4 CTAs (16 warps, 256 TMEM columns) per SM.
+// The tensor pipe is idle nine tenths of the time: building the operand rows and the GELU
+// epilogues bound the kernel by issue, so the epilogues use the packed FP32 instructions and the
+// rows are built from 32-bit words: 271 -> 252 us at 4400 x 640 on a B200.
 // ---------------------------------------------------------------------------
 constexpr int MT_Z = 32, MT_R = 4, MT_THREADS = 128;
 constexpr int MBOX_Z = MT_Z + 4, MBOX_R = MT_R + 4, MBOX_N = MBOX_Z * MBOX_R;  // 288 points
@@ -275,7 +306,7 @@ constexpr uint32_t M_OW1 = 0;
 constexpr uint32_t M_OW2 = M_OW1 + MLP_HID * MLP_K1 * 2;      // 14336
 constexpr uint32_t M_OA = M_OW2 + MLP_HID * MLP_HID * 2;      // 22528
 constexpr uint32_t M_OBOX = M_OA + MT_THREADS * MLP_K1 * 2;   // 51200
-constexpr uint32_t M_OP = M_OBOX + MLP_CH * MBOX_N * 2;       // 53504
+constexpr uint32_t M_OP = M_OBOX + 2 * MLP_CH * MBOX_N * 2;   // 55808 (the box and its shifted copy)
 constexpr uint32_t M_NP = MLP_HID + MLP_HID + MLP_OUT * MLP_HID + MLP_OUT;
 constexpr size_t M_SMEM = M_OP + M_NP * 4 + 128;  // + alignment slack
 constexpr int M_CTAS_PER_SM = 4;
@@ -358,10 +389,13 @@ __global__ void __launch_bounds__(MT_THREADS)
     for (int q = 0; q < MBOX_PER; ++q) {
       const int e = tid + q * MT_THREADS;
       if (e < MBOX_N) {
-        sBox[0 * MBOX_N + e] = __float2bfloat16_rn((v[q].x - a.norm.feat_mean[0]) * a.norm.feat_inv_scale[0]);
-        sBox[1 * MBOX_N + e] = __float2bfloat16_rn((v[q].y - a.norm.feat_mean[1]) * a.norm.feat_inv_scale[1]);
-        sBox[2 * MBOX_N + e] = __float2bfloat16_rn((v[q].z - a.norm.feat_mean[2]) * a.norm.feat_inv_scale[2]);
-        sBox[3 * MBOX_N + e] = __float2bfloat16_rn((v[q].w - a.norm.feat_mean[3]) * a.norm.feat_inv_scale[3]);
+        const float f[4] = {v[q].x, v[q].y, v[q].z, v[q].w};
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+          const __nv_bfloat16 x = __float2bfloat16_rn((f[ch] - a.norm.feat_mean[ch]) * a.norm.feat_inv_scale[ch]);
+          sBox[ch * MBOX_N + e] = x;
+          if (ch * MBOX_N + e > 0) sBox[MLP_CH * MBOX_N + ch * MBOX_N + e - 1] = x;  // the shifted copy
+        }
       }
     }
   };
@@ -386,26 +420,34 @@ __global__ void __launch_bounds__(MT_THREADS)
     const InferArgs& at = BATCH ? argv[inst] : a0;
     const Grid g = at.g;
     // A row `tid` of layer 1: feature k = ch*25 + (dr+2)*5 + (dz+2), zero for k >= 100
-    const unsigned short* bx = reinterpret_cast<const unsigned short*>(sBox);
+    // Five values from column c on per (channel, row) as three words: a second copy of the box
+    // one column further makes the words of odd columns aligned too.
+    const uint32_t* bw = reinterpret_cast<const uint32_t*>(sBox + (c & 1) * (MLP_CH * MBOX_N)) + rr * (MBOX_Z / 2) + (c >> 1);
+    auto words = [&](int gq, uint32_t (&w)[3]) {  // group gq = ch * 5 + dr
+      const uint32_t* q = bw + (gq / 5) * (MBOX_N / 2) + (gq % 5) * (MBOX_Z / 2);
+      w[0] = q[0];
+      w[1] = q[1];
+      w[2] = q[2];
+    };
+    uint32_t row[MLP_K1 / 2];
 #pragma unroll
-    for (int kc = 0; kc < MLP_K1 / 8; ++kc) {
-      uint32_t pk[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t hv[2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int k = kc * 8 + 2 * q + h;
-          hv[h] = 0u;
-          if (k < MLP_IN) {
-            const int ch = k / 25, w = k - ch * 25, dr = w / 5, dz = w - dr * 5;
-            hv[h] = bx[ch * MBOX_N + (rr + dr) * MBOX_Z + c + dz];
-          }
-        }
-        pk[q] = hv[0] | (hv[1] << 16);
-      }
-      *reinterpret_cast<uint4*>(base + M_OA + kmaj(tid, kc * 8, MT_THREADS)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+    for (int gq = 0; gq < MLP_IN / 5; gq += 2) {  // ten values, five words
+      uint32_t w[3], n[3];
+      words(gq, w);
+      words(gq + 1, n);
+      uint32_t* o = row + gq / 2 * 5;
+      o[0] = w[0];
+      o[1] = w[1];
+      o[2] = __byte_perm(w[2], n[0], 0x5410);  // low halves
+      o[3] = __byte_perm(n[0], n[1], 0x5432);  // high, low
+      o[4] = __byte_perm(n[1], n[2], 0x5432);
     }
+#pragma unroll
+    for (int e = MLP_IN / 2; e < MLP_K1 / 2; ++e) row[e] = 0u;
+#pragma unroll
+    for (int kc = 0; kc < MLP_K1 / 8; ++kc)
+      *reinterpret_cast<uint4*>(base + M_OA + kmaj(tid, kc * 8, MT_THREADS)) =
+          make_uint4(row[4 * kc], row[4 * kc + 1], row[4 * kc + 2], row[4 * kc + 3]);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -435,9 +477,12 @@ __global__ void __launch_bounds__(MT_THREADS)
     for (int q = 0; q < MLP_HID / 8; ++q) {
       uint32_t pk[4];
 #pragma unroll
-      for (int h = 0; h < 4; ++h)
-        pk[h] = pack_bf16(gelu_fast(z[q * 8 + 2 * h] + sB1[q * 8 + 2 * h]),
-                          gelu_fast(z[q * 8 + 2 * h + 1] + sB1[q * 8 + 2 * h + 1]));
+      for (int h = 0; h < 4; ++h) {
+        const int e = q * 8 + 2 * h;
+        float g0, g1;
+        unpk2(gelu_fast2(add2(pk2(z[e], z[e + 1]), *reinterpret_cast<const f32x2*>(sB1 + e))), g0, g1);
+        pk[h] = pack_bf16(g0, g1);
+      }
       *reinterpret_cast<uint4*>(base + M_OA + kmaj(tid, q * 8, MT_THREADS)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
     fence_async_smem();
@@ -462,13 +507,18 @@ __global__ void __launch_bounds__(MT_THREADS)
 #pragma unroll
     for (int q = 0; q < MLP_HID / 16; ++q) tmem_ld16(lane_base + q * 16, z + q * 16);
     tmem_wait_ld();
-    float y0 = sB3[0], y1 = sB3[1];
+    f32x2 a0 = pk2(sB3[0], 0.0f), a1 = pk2(sB3[1], 0.0f);
 #pragma unroll
-    for (int h = 0; h < MLP_HID; ++h) {
-      const float hv = gelu_fast(z[h] + sB2[h]);
-      y0 = fmaf(sW3[h], hv, y0);
-      y1 = fmaf(sW3[MLP_HID + h], hv, y1);
+    for (int h = 0; h < MLP_HID; h += 2) {
+      const f32x2 hv = gelu_fast2(add2(pk2(z[h], z[h + 1]), *reinterpret_cast<const f32x2*>(sB2 + h)));
+      a0 = fma2(*reinterpret_cast<const f32x2*>(sW3 + h), hv, a0);
+      a1 = fma2(*reinterpret_cast<const f32x2*>(sW3 + MLP_HID + h), hv, a1);
     }
+    float y0, y1, yo;
+    unpk2(a0, y0, yo);
+    y0 += yo;
+    unpk2(a1, y1, yo);
+    y1 += yo;
     tc_fence_before();
     const int i = i0 + c, j = j0 + rr;
     if (i < g.Nz && j < g.Nr) {
