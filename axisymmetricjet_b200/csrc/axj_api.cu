@@ -84,9 +84,8 @@ struct axj_handle {
   SideStream side{nullptr, nullptr, nullptr};  // general-tile launches run here, joined back
   std::string err;
   std::vector<void*> allocs;
-  // state and RK4 work buffers (5 planes each): the stage states; the running sum A and k2 B
-  // of the mixed path
-  double *U0 = nullptr, *Ua = nullptr, *Ub = nullptr, *Uc = nullptr, *A = nullptr, *B = nullptr, *target = nullptr;
+  // state and RK4 work buffers (5 planes each)
+  double *U0 = nullptr, *Ua = nullptr, *Ub = nullptr, *A = nullptr, *B = nullptr, *target = nullptr;
   // mixed precision: the intermediate stage states as FP32 planes (pitch P) in the
   // memory of Ua / Ub, which the unit entry points use as FP64 scratch
   float *Uaf = nullptr, *Ubf = nullptr;
@@ -157,17 +156,16 @@ struct axj_handle {
   bool out_pending = false;
   int64_t out_iter = 0;
   // TMA descriptors: stage-input halo boxes for the stage buffers x {interior, general}
-  // tiles, coefficient halo boxes, and tile boxes of pv_old, the running sum A and k2 (mixed)
-  // or the first and second stage states (FP64)
-  CUtensorMap map_state[6][2];
+  // tiles, coefficient halo boxes, and tile boxes of pv_old and the running sum A
+  CUtensorMap map_state[5][2];
   CUtensorMap map_star[2];
   CUtensorMap map_starL[2];    // final mu*, beta*, kappa* planes (learned sensor)
   CUtensorMap map_u0_tile, map_acc_tile, map_b_tile;
-  CUtensorMap map_sens[6][2];  // sensor V boxes of the stage buffers x {interior, general}
-  CUtensorMap map_sensT[6][2]; // sensor temperature boxes
+  CUtensorMap map_sens[5][2];  // sensor V boxes of the stage buffers x {interior, general}
+  CUtensorMap map_sensT[5][2]; // sensor temperature boxes
   // fused z/r filter: Q blocks, z and r code blocks, temperature blocks of the stage
   // buffers; the coefficient planes it writes, as boxes of the two tile classes
-  CUtensorMap map_zrQ, map_zrZc, map_zrRc, map_zrT[6];
+  CUtensorMap map_zrQ, map_zrZc, map_zrRc, map_zrT[5];
   std::vector<int2> zr_rb;      // its row blocks (zr_row_blocks) and segment length
   int2* zr_rblocks = nullptr;
   int zr_seg = ZRK_BZ;
@@ -175,20 +173,19 @@ struct axj_handle {
   // interior tiles as two CTAs of TR / 2 rows (int_rows == TR / 2, or a batch tuned so):
   // their boxes
   int int_rows = TR;
-  CUtensorMap map_stateH[6], map_starH, map_starLH, map_coefH, map_u0H, map_accH, map_bH;
+  CUtensorMap map_stateH[5], map_starH, map_starLH, map_coefH, map_u0H, map_accH, map_bH;
   CUtensorMap map_tgt, map_tgtH;  // pv_target tile boxes (L2 prefetch of the sponge tiles)
 };
 
 namespace {
-// Stage buffers by id: U0, Ua, Ub, Uc in FP64; Ua, Ub as FP32 planes (mixed path only).
-enum { BU0 = 0, BUA = 1, BUB = 2, BUC = 3, BUAF = 4, BUBF = 5, NBUF = 6 };
+// Stage buffers by id: U0, Ua, Ub in FP64; Ua, Ub as FP32 planes (mixed path only).
+enum { BU0 = 0, BUA = 1, BUB = 2, BUAF = 3, BUBF = 4, NBUF = 5 };
 inline bool buf_f32(int b) { return b >= BUAF; }
 inline void* buf_ptr(axj_handle* h, int b) {
   switch (b) {
     case BU0: return h->U0;
     case BUA: return h->Ua;
     case BUB: return h->Ub;
-    case BUC: return h->mixed ? h->A : h->Uc;  // (never a stage buffer of the mixed path)
     case BUAF: return h->Uaf;
     default: return h->Ubf;
   }
@@ -352,8 +349,6 @@ StageArgs stage_args(axj_handle* h, int bin, int bout, int stage) {
   a.U0 = h->U0;
   a.A = h->A;
   a.B = h->B;
-  a.U1 = h->mixed ? nullptr : h->Ua;
-  a.U2 = h->mixed ? nullptr : h->Ub;
   a.Uout = buf_f32(bout) ? nullptr : static_cast<double*>(buf_ptr(h, bout));
   a.Uout_f = buf_f32(bout) ? static_cast<float*>(buf_ptr(h, bout)) : nullptr;
   a.target = h->target;
@@ -501,9 +496,9 @@ int build_maps(axj_handle* h) {
   stage_boxes(false, h->mixed, &hw, &hh, &qh, &tw, &th, nullptr);
   int rc = make_map(h, &h->map_u0_tile, h->U0, 5, tw, th, 5);
   if (rc != AXJ_OK) return rc;
-  rc = make_map(h, &h->map_b_tile, h->mixed ? h->B : h->Ub, 5, tw, th, 5);
+  rc = make_map(h, &h->map_b_tile, h->B, 5, tw, th, 5);
   if (rc != AXJ_OK) return rc;
-  rc = make_map(h, &h->map_acc_tile, h->mixed ? h->A : h->Ua, 5, tw, th, 5);
+  rc = make_map(h, &h->map_acc_tile, h->A, 5, tw, th, 5);
   if (rc == AXJ_OK) rc = make_map(h, &h->map_tgt, h->target, 5, tw, th, 5);
   if (rc != AXJ_OK) return rc;
   // the half tiles of the interior class (a handle's int_rows, or a batch's tuning)
@@ -514,8 +509,8 @@ int build_maps(axj_handle* h) {
   if (rc == AXJ_OK) rc = make_map(h, &h->map_starH, h->Qz ? h->Qz : h->star, 3, hw, qh, 3);
   if (rc == AXJ_OK) rc = make_map(h, &h->map_starLH, h->star, 3, hw, qlh, 3);
   if (rc == AXJ_OK) rc = make_map(h, &h->map_u0H, h->U0, 5, tw, th, 5);
-  if (rc == AXJ_OK) rc = make_map(h, &h->map_bH, h->mixed ? h->B : h->Ub, 5, tw, th, 5);
-  if (rc == AXJ_OK) rc = make_map(h, &h->map_accH, h->mixed ? h->A : h->Ua, 5, tw, th, 5);
+  if (rc == AXJ_OK) rc = make_map(h, &h->map_bH, h->B, 5, tw, th, 5);
+  if (rc == AXJ_OK) rc = make_map(h, &h->map_accH, h->A, 5, tw, th, 5);
   if (rc == AXJ_OK) rc = make_map(h, &h->map_tgtH, h->target, 5, tw, th, 5);
   return rc;
 }
@@ -716,13 +711,10 @@ int enqueue_stage_learned(axj_handle* h, int bin, int bout, int stage, bool judg
   return launch_stage_kernels(h, bin, bout, stage, CM_LRN);
 }
 
-// Stage input/output buffers of RK4: U0 -> Ua -> Ub -> Uc -> U0, all three stage states kept
-// for the last update (FP64); U0 -> Ua -> Ub -> Ua -> U0 with FP32 Ua, Ub (mixed).
+// Stage input/output buffers of RK4: U0 -> Ua -> Ub -> Ua -> U0 (FP32 Ua, Ub when mixed).
 void rk4_buffers(const axj_handle* h, int b[5]) {
-  b[0] = b[4] = BU0;
-  b[1] = h->mixed ? BUAF : BUA;
-  b[2] = h->mixed ? BUBF : BUB;
-  b[3] = h->mixed ? BUAF : BUC;
+  const int a = h->mixed ? BUAF : BUA, c = h->mixed ? BUBF : BUB;
+  b[0] = BU0; b[1] = a; b[2] = c; b[3] = a; b[4] = BU0;
 }
 
 // ComputeTimeStep on the device; with advance != 0 the kernel also performs
@@ -1570,12 +1562,8 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
     h->Uaf = reinterpret_cast<float*>(h->Ua);
     h->Ubf = reinterpret_cast<float*>(h->Ub);
   }
-  if (h->mixed) {
-    h->A = dalloc<double>(h, 5 * pl, &rc);
-    h->B = dalloc<double>(h, 5 * pl, &rc);
-  } else {
-    h->Uc = dalloc<double>(h, 5 * pl, &rc);
-  }
+  h->A = dalloc<double>(h, 5 * pl, &rc);
+  h->B = dalloc<double>(h, 5 * pl, &rc);
   h->target = dalloc<double>(h, 5 * pl, &rc);
   h->star = dalloc<double>(h, 3 * pl, &rc);
   if (c.shock_capturing) {
@@ -2394,7 +2382,7 @@ struct axj_batch {
   // device tables
   CUtensorMap* maps = nullptr;
   StageArgs* stage_argv[3][5] = {};  // coefficient box CM_FILT, CM_LRN, CM_PRE
-  SensorArgs* sens_argv[NBUF] = {};
+  SensorArgs* sens_argv[5] = {};
   FeatArgs* feat_argv = nullptr;
   InferArgs* infer_argv[2] = {};
   JudgeArgs* judge_argv = nullptr;
@@ -2407,7 +2395,7 @@ struct axj_batch {
   ZrArgs* zr_argv = nullptr;
   int4* zr_items = nullptr;
   int nzr_items = 0;
-  SensorArgs a0_sens[NBUF];
+  SensorArgs a0_sens[5];
   InferArgs a0_infer[2];
   // host tile lists (i0, j0, instance) and their device copies
   std::vector<int4> h_st_int, h_st_gen, h_se_int, h_se_gen, h_ft, h_mt, h_st_half;
@@ -2692,8 +2680,8 @@ int batch_build_tables(axj_batch* b) {
       m[bmap_star(cls, false)] = h->map_star[cls];
       m[bmap_star(cls, true)] = h->map_starL[cls];
     }
-    m[bmap_u0] = h->map_u0_tile;
-    m[bmap_acc] = h->map_acc_tile;
+    m[14] = h->map_u0_tile;
+    m[15] = h->map_acc_tile;
     for (int bf = 0; bf < NBUF; ++bf) m[bmap_stateH(bf)] = h->map_stateH[bf < nb ? bf : 0];
     m[bmap_starH(false)] = h->map_starH;
     m[bmap_starH(true)] = h->map_starLH;

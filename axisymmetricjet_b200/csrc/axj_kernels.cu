@@ -313,28 +313,6 @@ __host__ __device__ constexpr int hz_t(int h, int esize) { return (h + 16 / esiz
 template <typename R, int TRT>
 __host__ __device__ constexpr bool rk_global() { return TRT < TR && sizeof(R) == 4; }
 
-// How RK4 combines its stages. FP64 stage states: the three of them stay in memory and the last
-// stage forms pv_old + (k1/2 + k2 + k3)/3 + k4/6 from their differences to pv_old, which are
-// exact; its one rounding per sum is no larger than the running sum's three. A step then moves
-// 520 B of state per point where the running sum and k2 took 640 (the third stage alone 240: it
-// read pv_old, the sum and k2 and wrote the sum and the state). Against extended precision a
-// step's rounding is 0.37 units in the last place rms, the running sum's 0.50. Measured on a
-// B200: the four interior launches of a 4400 x 640 step 540 -> 497 us (the third 151 -> 120), an
-// 1801 x 333 step 412 -> 385 us.
-// FP32 stage states (the mixed path) would lose the accumulation's FP64: running sum A and k2.
-template <typename R>
-__host__ __device__ constexpr bool rk_states() { return sizeof(R) == 8; }
-// Does the update of a stage read pv_old / the accumulator (mixed: A; FP64: the first state)?
-// (Stage 1 takes pv_old from its input box.)
-template <typename R>
-__host__ __device__ constexpr bool rk_reads_u0(int stage) {
-  return stage == 2 || stage == 3 || (rk_states<R>() && stage == 4);
-}
-template <typename R>
-__host__ __device__ constexpr bool rk_reads_acc(int stage) {
-  return stage == 4 || (!rk_states<R>() && stage == 3);
-}
-
 // TRT: rows of the tile (TR; interior tiles can also run as two halves of TR / 2 rows,
 // which need about half the shared memory and so let four to six CTAs share an SM).
 template <int H, typename SIN, typename R, int CM = CM_FILT, int TRT = TR>
@@ -442,8 +420,8 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
   // a double stage input with FP32 stencils is the mixed path's pv: stage 1, or the right-hand
   // side alone (stage 0); the later stages' code is left out of those instances
   constexpr bool FIRST = !std::is_same<SIN, R>::value;
-  const bool needU0 = !FIRST && !RKG && rk_reads_u0<R>(a.stage);
-  const bool needA = !FIRST && !RKG && rk_reads_acc<R>(a.stage);
+  const bool needU0 = !FIRST && !RKG && (a.stage == 2 || a.stage == 3);
+  const bool needA = !FIRST && !RKG && (a.stage == 3 || a.stage == 4);
   // mu = T**0.666 (AssignValues) on the cross of the region (CM_PRE: the coefficient box
   // already holds mu_eff, beta and kappa_eff). With shock capturing the
   // coefficient box holds the z-filtered quantities; the r filter PerformTGfilter(q, 2,
@@ -700,16 +678,9 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       const long long o = f * PL + go;
       u0v[f] = av[f] = bv[f] = 0.0;
       if (FIRST) continue;
-      if (rk_reads_u0<R>(a.stage)) u0v[f] = RKG ? a.U0[o] : sP0[f * NTP + tp];
-      if constexpr (rk_states<R>()) {
-        if (a.stage == 4) {
-          av[f] = RKG ? __ldg(a.U1 + o) : sPA[f * NTP + tp];
-          bv[f] = __ldg(a.U2 + o);
-        }
-      } else {
-        if (a.stage == 3 || a.stage == 4) av[f] = RKG ? a.A[o] : sPA[f * NTP + tp];
-        if (a.stage == 3) bv[f] = __ldg(a.B + o);
-      }
+      if (a.stage == 2 || a.stage == 3) u0v[f] = RKG ? __ldg(a.U0 + o) : sP0[f * NTP + tp];
+      if (a.stage == 3 || a.stage == 4) av[f] = RKG ? a.A[o] : sPA[f * NTP + tp];
+      if (a.stage == 3) bv[f] = __ldg(a.B + o);
     }
     // pv_target is read only where a term uses it: sponges, face operations, forcing
     const bool need_tg = (rloc >= a.c.sponge_start_top) || (!j1 && zloc <= a.c.sponge_end_left) ||
@@ -747,20 +718,13 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       if (FIRST || a.stage == 1) {
         const double u0 = pv[f];  // pv_old = stage-1 input
         un[f] = add_rn(u0, mul_rn(0.5, k));
-        if constexpr (!rk_states<R>()) a.A[o] = add_rn(u0, mul_rn(c6, k));
+        a.A[o] = add_rn(u0, mul_rn(c6, k));
       } else if (a.stage == 2) {
         un[f] = add_rn(u0v[f], mul_rn(0.5, k));
-        if constexpr (!rk_states<R>()) a.B[o] = k;
+        a.B[o] = k;
       } else if (a.stage == 3) {
         un[f] = add_rn(u0v[f], k);
-        if constexpr (!rk_states<R>()) a.A[o] = add_rn(av[f], mul_rn(c3, add_rn(bv[f], k)));
-      } else if constexpr (rk_states<R>()) {
-        // pv_old + (k1/2 + k2 + k3)/3 + k4/6 with k1/2, k2/2, k3 as the differences of the stage
-        // states (exact: neighbouring values) from pv_old; this stage's input is the third
-        const double u0 = u0v[f];
-        const double d = add_rn(add_rn(av[f], -u0), add_rn(pv[f], -u0));
-        const double q = add_rn(d, mul_rn(2.0, add_rn(bv[f], -u0)));
-        un[f] = blank ? pv[f] : add_rn(u0, add_rn(mul_rn(c3, q), mul_rn(c6, k)));
+        a.A[o] = add_rn(av[f], mul_rn(c3, add_rn(bv[f], k)));
       } else {
         un[f] = blank ? pv[f] : add_rn(av[f], mul_rn(c6, k));
       }
@@ -819,12 +783,12 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
     nrow = TRT - (j0 >> 24);
     j0 &= 0xFFFFFF;
   }
-  // the RK operands of this stage (rk_states): interior tiles stage two of them by TMA; general
-  // tiles and FP32 half tiles read them from global memory
+  // pv_old is needed as a tile in stages 2 and 3 (stage 1 reads it from the state box),
+  // the running sum A in stages 3 and 4; interior tiles stage them by TMA
+  // RK operands from global memory (general tiles, FP32 half tiles) or staged by TMA
   constexpr bool RKG = GEN || rk_global<R, TRT>();
-  const bool readU0 = rk_reads_u0<R>(a.stage), readA = rk_reads_acc<R>(a.stage);
-  const bool needU0 = !RKG && readU0;
-  const bool needA = !RKG && readA;
+  const bool needU0 = !RKG && (a.stage == 2 || a.stage == 3);
+  const bool needA = !RKG && (a.stage == 3 || a.stage == 4);
 
   // ---- phase 1: one thread issues the TMA loads; the RK operands complete on the
   // second barrier while phases 1-2 run. The barriers are initialised once per CTA by the
@@ -842,9 +806,9 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
       if (needU0) tma_load_3d(sP0, mU0, i0, j0, 0, &bar[1]);
       if (needA) tma_load_3d(sPA, mAcc, i0, j0, 0, &bar[1]);
     }
-    // operands the RK update reads from global memory: into L2 now (k2 in stage 3 or the second
-    // stage state in stage 4; the others where they are not staged)
-    if (mB && a.stage == (rk_states<R>() ? 4 : 3)) tma_prefetch_3d(mB, i0, j0, 0);
+    // operands the RK update reads from global memory: into L2 now (k2 in stage 3; pv_old
+    // and the running sum in general tiles, which do not stage them)
+    if (mB && a.stage == 3) tma_prefetch_3d(mB, i0, j0, 0);
     // pv_target, which the sponges (and the face operations, the feedback forcing) read per
     // point from global memory: into L2 for the tiles that reach a sponge
     if (mTg) {
@@ -852,8 +816,8 @@ __device__ __forceinline__ bool stage_body(const StageArgs& a, int i0, int j0, c
                        __ldg(a.rc + min(j0 + TRT - 1, Nr - 1)) >= a.c.sponge_start_top;
       if (tgt) tma_prefetch_3d(mTg, i0, j0, 0);
     }
-    if (RKG && readU0) tma_prefetch_3d(mU0, i0, j0, 0);
-    if (RKG && readA) tma_prefetch_3d(mAcc, i0, j0, 0);
+    if (RKG && (a.stage == 2 || a.stage == 3)) tma_prefetch_3d(mU0, i0, j0, 0);
+    if (RKG && (a.stage == 3 || a.stage == 4)) tma_prefetch_3d(mAcc, i0, j0, 0);
   }
   // the tile's metrics and coordinates (read per point in phases 2-3)
   if (tid < TZ) {
@@ -2850,7 +2814,7 @@ static cudaError_t launch_stage_batch_t(const StageArgs* argv, const BatchTiles&
   int4 k;
   if (TRT == TR) {
     const int star = CM == CM_PRE ? bmap_coef(cls) : bmap_star(cls, CM == CM_LRN);
-    k = make_int4(bmap_state(kin, cls), star, bmap_u0, bmap_acc);
+    k = make_int4(bmap_state(kin, cls), star, 14, 15);
   } else {
     const int star = CM == CM_PRE ? bmap_coef(2) : bmap_starH(CM == CM_LRN);
     k = make_int4(bmap_stateH(kin), star, bmap_u0H, bmap_accH);

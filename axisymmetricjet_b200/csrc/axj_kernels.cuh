@@ -11,13 +11,13 @@ namespace axj {
 
 // TMA descriptors of one fused-stage launch: the stage input with its halo box for
 // the tile class, the shock-capturing coefficient planes with the same box, and
-// the tile-sized boxes of pv_old and the running RK sum (FP64: the first stage state).
+// the tile-sized boxes of pv_old and the running RK sum.
 struct StageMaps {
   const CUtensorMap* state;
   const CUtensorMap* star;
   const CUtensorMap* u0;
   const CUtensorMap* acc;
-  const CUtensorMap* bt;  // tile box of k2 (prefetched into L2 for stage 3), FP64: of the second stage state (stage 4)
+  const CUtensorMap* bt;  // tile box of k2 (prefetched into L2 for stage 3)
   const CUtensorMap* tg;  // tile box of pv_target (prefetched into L2 where sponges or faces read it)
 };
 
@@ -41,10 +41,8 @@ struct StageArgs {
   Grid g;
   const double* Uin;     // stage input state (5 planes)
   const double* U0;      // pv_old (5 planes)
-  double* A;             // mixed path: running sum  pv_old + k1/6 (+ (k2+k3)/3)
-  double* B;             // mixed path: k2
-  const double* U1;      // FP64 path: the first and second stage states (read in stage 4)
-  const double* U2;
+  double* A;             // running sum  pv_old + k1/6 (+ (k2+k3)/3)
+  double* B;             // k2
   double* Uout;          // stage output (5 planes); rhs (5 planes) in stage 0
   float* Uout_f;         // FP32 stage output (mixed precision, stages 1-3)
   const double* target;  // pv_target (5 planes)
@@ -219,29 +217,28 @@ cudaError_t launch_tgfilter_z_inplace(const Grid& g, const uint32_t* desc, const
 
 // ---- batched launches: many solver instances per launch ----
 // Per-instance TMA maps of a batch, NM_BATCH per instance, at these indices:
-//   state box of stage buffer b (0..5), tile class cls:  b * 2 + cls  (0..11)
-//   z-filtered coefficient box of class cls:       12 + cls
-//   final-coefficient box of class cls:            14 + cls
-//   pv_old tile box, running-sum (FP64: first stage state) tile box: 16, 17
-//   sensor V box of buffer b, class cls:           18 + b * 2 + cls  (18..29)
-//   sensor temperature box of buffer b, class cls: 30 + b * 2 + cls  (30..41)
-//   interior half tiles (TR / 2 rows): state box of buffer b 42 + b (42..47), z-filtered
-//   coefficient box 48, final-coefficient box 49, pv_old and running-sum tile boxes 50, 51
-//   fused z/r filter: Q blocks 52, z and r code blocks 53, 54, temperature blocks of
-//   buffer b 55 + b (55..60); its coefficient planes as boxes of the interior, general and
-//   half tiles 61, 62, 63
-constexpr int NM_BATCH = 64;
+//   state box of stage buffer b, tile class cls:  b * 2 + cls         (0..9)
+//   z-filtered coefficient box of class cls:      10 + cls
+//   final-coefficient box of class cls:           12 + cls
+//   pv_old tile box, running-sum tile box:         14, 15
+//   sensor V box of buffer b, class cls:           16 + b * 2 + cls  (16..25)
+//   sensor temperature box of buffer b, class cls: 26 + b * 2 + cls  (26..35)
+//   interior half tiles (TR / 2 rows): state box of buffer b 36 + b (36..40), z-filtered
+//   coefficient box 41, final-coefficient box 42, pv_old and running-sum tile boxes 43, 44
+//   fused z/r filter: Q blocks 45, z and r code blocks 46, 47, temperature blocks of
+//   buffer b 48 + b (48..52); its coefficient planes as boxes of the interior, general and
+//   half tiles 53, 54, 55
+constexpr int NM_BATCH = 56;
 inline int bmap_state(int b, int cls) { return b * 2 + cls; }
-inline int bmap_star(int cls, bool lrn) { return (lrn ? 14 : 12) + cls; }
-constexpr int bmap_u0 = 16, bmap_acc = 17;
-inline int bmap_sens(int b, int cls) { return 18 + b * 2 + cls; }
-inline int bmap_sensT(int b, int cls) { return 30 + b * 2 + cls; }
-inline int bmap_stateH(int b) { return 42 + b; }
-inline int bmap_starH(bool lrn) { return lrn ? 49 : 48; }
-constexpr int bmap_u0H = 50, bmap_accH = 51;
-constexpr int bmap_zrQ = 52, bmap_zrZc = 53, bmap_zrRc = 54;
-inline int bmap_zrT(int b) { return 55 + b; }
-inline int bmap_coef(int cls) { return 61 + cls; }  // cls 0 interior, 1 general, 2 half tiles
+inline int bmap_star(int cls, bool lrn) { return (lrn ? 12 : 10) + cls; }
+inline int bmap_sens(int b, int cls) { return 16 + b * 2 + cls; }
+inline int bmap_sensT(int b, int cls) { return 26 + b * 2 + cls; }
+inline int bmap_stateH(int b) { return 36 + b; }
+inline int bmap_starH(bool lrn) { return lrn ? 42 : 41; }
+constexpr int bmap_u0H = 43, bmap_accH = 44;
+constexpr int bmap_zrQ = 45, bmap_zrZc = 46, bmap_zrRc = 47;
+inline int bmap_zrT(int b) { return 48 + b; }
+inline int bmap_coef(int cls) { return 53 + cls; }  // cls 0 interior, 1 general, 2 half tiles
 
 struct BatchTiles {
   const int4* tiles;  // (i0, j0, instance, 0)
