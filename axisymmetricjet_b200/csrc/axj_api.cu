@@ -580,12 +580,13 @@ std::vector<int2> zr_row_blocks(const std::vector<unsigned char>& rcode, int Nz,
 }
 
 // Segment length (z positions) of the fused z/r filter over work items of Nz positions x
-// row blocks. A CTA's time goes with its blocks of 16 positions plus 2.5 (its warm-up blocks
+// row blocks. A CTA's time goes with its blocks of 16 positions plus 2.5 (its four warm-up blocks
 // run the recurrence alone); two CTAs of an SM take 1.03, three 1.2 times one's time, and more
 // than three run in turns. So small grids take the shortest segments that fill the SMs once and
-// large ones the longest that still leave three CTAs for each SM. Measured on a B200 (16 / 32 / 48
-// positions): 787 x 203 15.4 / 18.2 / 21.0 us; 1801 x 333 29.9 / 27.2 / 21.0, 64: 21.2;
-// 4400 x 640 176: 56.6, 96: 64, 272: 73.
+// large ones the longest that still leave three CTAs for each SM. Measured on a B200, the picked
+// length first: 787 x 203 16: 15.1 us (32: 17.7, 64: 25.1); 1024 x 256 32: 14.6 (16: 18.9, 48: 17.7);
+// 1801 x 333 48: 21.4 (32: 27.0, 64: 21.2); 2401 x 500 80: 29.6 (64: 37.4, 96: 31.2); 4400 x 640 176:
+// 55.8 (96: 64.7, 272: 68.1).
 int zr_pick_segment(const std::vector<std::pair<int, int>>& work, int nsm) {
   int kmax = 1;
   for (const auto& w : work) kmax = std::max(kmax, (w.first + ZRK_BZ - 1) / ZRK_BZ);

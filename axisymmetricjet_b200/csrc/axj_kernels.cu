@@ -2194,7 +2194,7 @@ __global__ void tgfilter_z_rows_kernel_batch(const SensorArgs* __restrict__ argv
 // side that the r filter reads: one thread per (quantity, row), marching along z in blocks of
 // ZRK_BZ positions. Segments start ZRK_WARM positions early from a zero history (the
 // recurrence forgets its start: the dominant root of its feedback part is about 0.47, so
-// 0.47**48 < 2e-16); the first segment starts exactly at i = 0 from the reference's zero
+// 0.47**64 = 1e-21); the first segment starts exactly at i = 0 from the reference's zero
 // halo. The z-filtered block goes to shared memory, where the r filter
 // PerformTGfilter(q, 2, star) of the CTA's rows is applied with the point's r row, then
 // the C*Re(*Pr) scaling, the z ramp and mu = T**0.666 of the stage input. A thread takes the
