@@ -161,8 +161,9 @@ __device__ __forceinline__ R dot_c1_p(const S* rho, const S* T, int stride) {
 
 // A stencil row as six taps (general tiles): the weights of both operators, the window's start
 // and the sixth tap's offset. Every row fits: the centred row's sixth weight is zero (that tap
-// reads the point itself), row 9 (no derivative) has zero weights. Read from a table in shared
-// memory [ROW6_ROWS][12], so lanes of a warp with different rows take one path.
+// reads the point itself), row 9 (no derivative) has zero weights: zero for any finite field
+// (products of fields may overflow, so their callers mask that row). Read from a table in
+// shared memory [ROW6_ROWS][12], so lanes of a warp with different rows take one path.
 constexpr int ROW6_ROWS = 10;
 template <typename R>
 struct Row6 {
@@ -598,7 +599,8 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       dr.dVtdz = dst6<R, C, 1>(q, pVt, 1) * xz;
       dr.dVzdz = sDz[RR * TZ + dzi];
       dr.dTdz = dst6<R, C, 1>(q, pT, 1) * xz;
-      dr.dpdz = dst6_p<R, C>(q, pR, pT, 1) * xz;
+      // (a blanked point's products may overflow where its values do not: zero times infinity)
+      dr.dpdz = C || zr < 9 ? dst6_p<R, C>(q, pR, pT, 1) * xz : R(0);
       dr.d2Vrdz2 = dst6<R, C, 2>(q, pVr, 1) * (xz * xz) + dr.dVrdz * xzz;
       dr.d2Vtdz2 = dst6<R, C, 2>(q, pVt, 1) * (xz * xz) + dr.dVtdz * xzz;
       dr.d2Vzdz2 = dst6<R, C, 2>(q, pVz, 1) * (xz * xz) + dr.dVzdz * xzz;
@@ -615,7 +617,7 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       dr.dVtdr = dst6<R, C, 1>(q, pVt, RZ) * er;
       dr.dVzdr = dst6<R, C, 1>(q, pVz, RZ) * er;
       dr.dTdr = dst6<R, C, 1>(q, pT, RZ) * er;
-      dr.dpdr = dst6_p<R, C>(q, pR, pT, RZ) * er;
+      dr.dpdr = C || rw < 9 ? dst6_p<R, C>(q, pR, pT, RZ) * er : R(0);
       dr.d2Vrdr2 = dst6<R, C, 2>(q, pVr, RZ) * (er * er) + dr.dVrdr * err;
       dr.d2Vtdr2 = dst6<R, C, 2>(q, pVt, RZ) * (er * er) + dr.dVtdr * err;
       dr.d2Vzdr2 = dst6<R, C, 2>(q, pVz, RZ) * (er * er) + dr.dVzdr * err;
