@@ -45,8 +45,10 @@ __device__ __forceinline__ double na_warp_min(double v) {
 
 // Per-point dt of ComputeTimeStep (ModInputOutput.f90:395-416), block minimum, and the
 // last block to finish reduces the per-block minima. A block takes one strip per warp
-// of the shared point scan (axj_dt.cuh); the largest rate is the smallest dt only for a positive CFL, so
-// any other CFL turns the scan's screening off.
+// of the shared point scan (axj_dt.cuh). The largest rate is the smallest dt only for a positive
+// CFL, and the estimate's viscous part is the rate's only for positive Re and Pr (dt_point takes the
+// largest of the quotients, of which a negative Re makes another one than the estimate's):
+// anything else, NaN among it, turns the screening off.
 template <bool SCREEN>
 __global__ void __launch_bounds__(NA_THREADS, 4)
     dt_noalloc_kernel(const double* __restrict__ U, long long P, long long plane, int Nz, int Nr,
@@ -184,7 +186,7 @@ extern "C" int axj_compute_dt_noalloc(const double* d_pv, int64_t pitch, int64_t
   cudaError_t e = cudaMemsetAsync(scratch + NA_COUNTER, 0, 2 * sizeof(double), s);
   if (e == cudaSuccess) {
     const long long n = Nz * Nr;
-    const bool screen = axj::dt_screened(n) && c.CFL > 0.0;
+    const bool screen = axj::dt_screened(n) && c.CFL > 0.0 && c.Re > 0.0 && c.Pr > 0.0;
     const long long need = axj::dt_blocks((int)Nz, (int)Nr, screen);
     const int blocks = (int)(need < NA_MAX_BLOCKS ? need : NA_MAX_BLOCKS);
     auto kernel = screen ? dt_noalloc_kernel<true> : dt_noalloc_kernel<false>;

@@ -1,0 +1,59 @@
+"""Inputs outside the range in which the FP32 estimate of the screened time-step scan bounds a
+point's rate: the scan has to evaluate such points in FP64, on grids large enough to be screened
+as on small ones. Oracle: the formula of ModInputOutput.f90:395-416 over every point in NumPy (64
+bits). Tolerance: as for the scan itself, 1e-14 (a rate is a sum of three terms of at most eight
+roundings each, plus a power within 2 ulp; the difference lambda = 0.6 mu - 2/3 mu loses one
+digit of its part)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import axisymmetricjet_b200 as axj
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-14
+SIZES = [(257, 13), (450, 311)]  # below and above 98,304 points
+
+
+def _call(pv, dxidz, detadr, params, stale=1.0):
+    import torch
+    fn = axj.load_library().axj_compute_dt_noalloc
+    fn.restype = C.c_int
+    fn.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
+                   C.POINTER(axj.AxjParams), C.c_double, C.c_void_p, C.c_void_p]
+    _, Nr, Nz = pv.shape
+    d, x, y = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (pv, dxidz, detadr))
+    dt = torch.zeros(1, dtype=torch.float64, device="cuda")
+    rc = fn(d.data_ptr(), Nz, Nz, Nr, x.data_ptr(), y.data_ptr(), None, C.byref(params), stale, dt.data_ptr(),
+            torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    return float(dt.item())
+
+
+def _dts(pv, dxidz, detadr, p, stale=None):
+    x, y = dxidz[None, :], detadr[:, None]
+    T = pv[4]
+    mu = T ** 0.666
+    lam = 0.6 * mu - 2.0 / 3.0 * mu
+    inv = np.abs(pv[3] * x + pv[1] * y) + np.sqrt(T if stale is None else stale) * np.sqrt(x * x + y * y)
+    m = np.maximum(np.maximum(mu / p.Re, lam / p.Re), mu / (p.Re * p.Pr))
+    return p.CFL / (inv + 2.0 * m * (np.abs(x) + np.abs(y)) ** 2)
+
+
+def _flow(Nz, Nr, seed=3):
+    rng = np.random.default_rng(seed)
+    pv = np.ones((5, Nr, Nz))
+    pv[1], pv[3] = rng.standard_normal((2, Nr, Nz))
+    pv[4] = rng.uniform(0.3, 3.0, (Nr, Nz))
+    return pv, rng.uniform(1.0, 80.0, Nz), rng.uniform(1.0, 200.0, Nr)
+
+
+@pytest.mark.parametrize("Nz,Nr", SIZES)
+@pytest.mark.parametrize("Re,Pr", [(-50.0, 0.72), (50.0, -0.72), (-50.0, -0.72), (-50.0, 100.0)])
+def test_negative_reynolds_or_prandtl_number(Nz, Nr, Re, Pr):
+    """The viscous part's maximum is then another of its terms than the estimate's."""
+    pv, dxidz, detadr = _flow(Nz, Nr)
+    p = axj.default_params(dt_mode=1, Re=Re, Pr=Pr)
+    want = _dts(pv, dxidz, detadr, p).min()
+    assert abs(_call(pv, dxidz, detadr, p) - want) <= TOL * abs(want)
