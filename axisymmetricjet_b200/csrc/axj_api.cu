@@ -735,6 +735,7 @@ DtArgs dt_args(axj_handle* h, int advance) {
   d.time = h->time;
   d.advance = advance;
   d.nblk = h->dt_blocks;
+  d.screen = dt_grid_screened(h->Nz, h->Nr, h->c);
   d.c = h->c;
   return d;
 }
@@ -1600,7 +1601,7 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
   h->harm = dalloc<double>(h, 5, &rc);
 
   h->counter = dalloc<unsigned int>(h, 2, &rc);
-  h->dt_blocks = dt_grid_blocks((int)Nz, (int)Nr);
+  h->dt_blocks = dt_grid_blocks((int)Nz, (int)Nr, h->c);
   h->partial = dalloc<double>(h, h->dt_blocks, &rc);
   h->tiles_int = dalloc<int2>(h, std::max<size_t>(tint.size(), 1), &rc);
   h->tiles_gen = dalloc<int2>(h, std::max<size_t>(tgen.size(), 1), &rc);

@@ -1053,13 +1053,16 @@ __device__ __forceinline__ double warp_min(double v) {
 // reduces x and divides once. Likewise max(mu/Re, lambda/Re) = max(mu, lambda)/Re. The
 // divisions by Re and Re Pr are products with the host's reciprocals (within an ulp of the
 // quotients). Blanked points contribute dt = 100
-// (ModInputOutput.f90:398-400).
+// (ModInputOutput.f90:398-400). Without a positive CFL the smallest dt is not at the largest x: the
+// kernel then divides at every point, unscreened, and xm is the maximum of -dt.
 template <bool SCREEN>
 __device__ __forceinline__ void dt_body(const DtArgs& a, int blk) {
   const long long PL = a.g.plane;
   const bool phys = a.c.dt_mode == DT_PHYSICAL;
   const double Tst = *a.staleT;
-  double xm = 0.0;  // maximum of the denominators (0: no unblanked point evaluated yet)
+  const bool pos = SCREEN || a.c.CFL > 0.0;
+  const double xm0 = pos ? 0.0 : -1.0e300;  // no unblanked point evaluated yet
+  double xm = xm0;                          // maximum of the denominators
   int bad = 0, blank = 0;
   __shared__ double sred[DT_THREADS / 32];
   __shared__ bool last;
@@ -1098,7 +1101,7 @@ __device__ __forceinline__ void dt_body(const DtArgs& a, int blk) {
           const double sabs = fabs(dxidz) + fabs(detadr);
           const double x = inv + 2.0 * mx * (sabs * sabs);
           if (!isfinite(x)) bad = 1;  // NaN, or an infinite input (which would give dt = 0)
-          xm = fmax(xm, x);
+          xm = fmax(xm, pos ? x : -(a.c.CFL / x));
         });
   const bool anyblank = __syncthreads_or(blank);
   xm = warp_max(xm);
@@ -1107,11 +1110,11 @@ __device__ __forceinline__ void dt_body(const DtArgs& a, int blk) {
   if (bad) atomicOr(a.flags, 1);
   __syncthreads();
   if (w == 0) {
-    xm = lane < DT_THREADS / 32 ? sred[lane] : 0.0;
+    xm = lane < DT_THREADS / 32 ? sred[lane] : xm0;
     xm = warp_max(xm);
     if (lane == 0) {
       // per-block dt (CFL / its largest denominator; 100 if it only met blanked points)
-      double v = a.c.CFL / xm;
+      double v = pos ? a.c.CFL / xm : -xm;
       if (anyblank) v = fmin(v, 100.0);
       a.partial[blk] = v;
       __threadfence();
@@ -1151,7 +1154,7 @@ __global__ void __launch_bounds__(DT_THREADS, 4) dt_kernel_batch(const DtArgs* _
   for (int k = threadIdx.x; k < (int)(sizeof(DtArgs) / 8); k += blockDim.x)
     reinterpret_cast<unsigned long long*>(&sa)[k] = reinterpret_cast<const unsigned long long*>(argv + blockIdx.y)[k];
   __syncthreads();
-  if (dt_screened((long long)sa.g.Nz * sa.g.Nr)) dt_body<true>(sa, blockIdx.x);
+  if (sa.screen) dt_body<true>(sa, blockIdx.x);
   else dt_body<false>(sa, blockIdx.x);
 }
 
@@ -1173,14 +1176,16 @@ cudaError_t launch_harmonic_phase(const double* time, const double* dt, double o
   return cudaGetLastError();
 }
 
-// Blocks of the dt kernel for the current device: as many as are resident at once (one
-// wave, every SM full), so that every thread's loads are in flight together.
-int dt_grid_blocks(int Nz, int Nr) {
-  return (int)std::min<long long>(dt_blocks(Nz, Nr, dt_screened((long long)Nz * Nr)), DT_MAX_BLOCKS);
+bool dt_grid_screened(int Nz, int Nr, const Consts& c) { return dt_screened((long long)Nz * Nr) && c.CFL > 0.0; }
+
+// Blocks of the dt kernel: one resident wave of a screened scan, else one strip row per warp, as far
+// as there are places for their minima (the blocks loop).
+int dt_grid_blocks(int Nz, int Nr, const Consts& c) {
+  return (int)std::min<long long>(dt_blocks(Nz, Nr, dt_grid_screened(Nz, Nr, c)), DT_MAX_BLOCKS);
 }
 
 cudaError_t launch_dt(const DtArgs& a, cudaStream_t s) {
-  if (dt_screened((long long)a.g.Nz * a.g.Nr)) dt_kernel<true><<<a.nblk, DT_THREADS, 0, s>>>(a);
+  if (a.screen) dt_kernel<true><<<a.nblk, DT_THREADS, 0, s>>>(a);
   else dt_kernel<false><<<a.nblk, DT_THREADS, 0, s>>>(a);
   return cudaGetLastError();
 }

@@ -89,6 +89,7 @@ struct DtArgs {
   double* time;          // solution time, advanced by dt when advance != 0
   int advance;
   int nblk;              // blocks of the instance (dt_grid_blocks)
+  int screen;            // whether its scan is screened (dt_grid_screened)
   Consts c;
 };
 
@@ -152,9 +153,10 @@ void stage_boxes(bool gen, bool mixed, int* halo_w, int* halo_h, int* q_h, int* 
 // V_r / V_z box vw x vh, temperature box tw x th (rho uses the stage tile box).
 void sensor_boxes(bool gen, bool mixed, int* vw, int* vh, int* tw, int* th);
 cudaError_t launch_dt(const DtArgs& a, cudaStream_t s);
-// Blocks of ComputeTimeStep over a grid (axj_dt.cuh): at most DT_MAX_BLOCKS; they loop over
-// its strips of points.
-int dt_grid_blocks(int Nz, int Nr);
+// Whether ComputeTimeStep over a grid is screened (axj_dt.cuh), and its blocks: at most
+// DT_MAX_BLOCKS; they loop over the grid's strips of points.
+bool dt_grid_screened(int Nz, int Nr, const Consts& c);
+int dt_grid_blocks(int Nz, int Nr, const Consts& c);
 // cos(omega t_s) of the harmonic forcing: rhs_mode != 0: out[0] at t = *time; else
 // out[s], s = 1..4, at t_s = (*time - *dt) + c_s * *dt (the device time is t_n + dt).
 cudaError_t launch_harmonic_phase(const double* time, const double* dt, double omega, int rhs_mode, double* out,

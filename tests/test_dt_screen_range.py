@@ -57,3 +57,22 @@ def test_negative_reynolds_or_prandtl_number(Nz, Nr, Re, Pr):
     p = axj.default_params(dt_mode=1, Re=Re, Pr=Pr)
     want = _dts(pv, dxidz, detadr, p).min()
     assert abs(_call(pv, dxidz, detadr, p) - want) <= TOL * abs(want)
+
+
+@pytest.mark.parametrize("Nz,Nr", [(48, 40), (450, 311)])
+@pytest.mark.parametrize("CFL", [-0.5, 0.0])
+def test_handle_without_a_positive_cfl(oracle_mod, Nz, Nr, CFL):
+    """dt = CFL / x is then not smallest where x is largest; the two entry points agree."""
+    from axisymmetricjet_b200 import fixtures
+    c = fixtures.make_case(Nz, Nr, 30.0, 15.0, 0.9, 1000.0, dt_mode=1, CFL=CFL)
+    c["pv"][1] += 0.1 * np.random.default_rng(3).standard_normal((Nr, Nz))
+    p = axj.patches_from_records(c["records"], Nz, Nr)
+    with axj.AxiJetSolver(c["params"], c["zvec"], c["rvec"], c["ibval"], p) as s:
+        ora = oracle_mod.Oracle(c["params"], c["zvec"], c["rvec"], c["ibval"], p)
+        s.set_state(c["pv"], c["target"])
+        ora.set_state(c["pv"], c["target"])
+        want = ora.compute_time_step()
+        assert abs(s.compute_time_step() - want) <= TOL * abs(want)
+        mz, mr = ora.metrics()[:2]
+        got = _call(c["pv"], np.ascontiguousarray(mz[0]), np.ascontiguousarray(mr[:, 0]), c["params"])
+        assert abs(got - want) <= TOL * abs(want)
