@@ -10,10 +10,10 @@
 // x in FP64 only where the estimate lies within DT_SCREEN of the parts' magnitudes of that.
 // The margin is an order of magnitude wider than the estimate's error, so the point of the
 // largest x is always among them and the result is the full FP64 scan's, bit for bit.
-// Estimates that are not finite (NaN or infinite inputs, FP32 overflow) are always evaluated
-// in FP64. The largest lower bound seen so far is handed from block to block through a word
-// in global memory (a hint: any value it holds is a valid bound), so that most blocks evaluate
-// no point in FP64 at all.
+// Estimates that are not finite (NaN or infinite inputs, FP32 overflow) and points where FP32
+// underflows (below) are always evaluated in FP64. The largest lower bound seen so far is handed
+// from block to block through a word in global memory (a hint: any value it holds is a valid
+// bound), so that most blocks evaluate no point in FP64 at all.
 // Measured at 4400 x 640 on a B200: the allocation-free kernel 51.4 -> 19.7 us (a call 57.4 ->
 // 22.6 us), the handle's 35.7 -> 23.0 us; what remains is issue (62 % of the active cycles) and
 // the launch's head and tail. Unscreened at 512 x 128 (one strip row per warp, a grid sized to
@@ -50,7 +50,15 @@ __host__ __device__ inline long long dt_blocks(int Nz, int Nr, bool screen) {
   return screen && b > DT_WAVE ? DT_WAVE : b;
 }
 constexpr float DT_SCREEN = 1.220703125e-4f;   // 2**-13
-constexpr float DT_TINY = 1.0e-30f;            // absolute margin (FP32 underflow, flushed subnormals)
+constexpr float DT_TINY = 1.0e-30f;            // absolute margin (subnormal products)
+// Underflow: the approximate units flush subnormals, so a T, or a sum of squared metrics, below FP32's
+// normal range loses its part of the estimate, and a T that is negative but small is no NaN. Either
+// makes mu * sqrt(g2) zero, and the point is then evaluated in FP64 whatever its estimate (which,
+// being too small, is still a valid lower bound). With both normal, what else underflows is below
+// the margin, for velocities up to 1e15 or metrics that are zero or normal in FP32; the stale T and
+// the viscous factors are tested once per launch (dt_factors). Overflow needs no test: an
+// infinite estimate is evaluated too.
+constexpr float DT_NORMAL = 1.17549435e-38f;
 
 __device__ __forceinline__ float f_sqrt(float x) {
   float y;
@@ -76,7 +84,16 @@ struct DtScan {
   const double* detadr;
   bool phys;     // sound speed from the point's T (else sqrt_stale)
   float sqrt_stale, inv_Re, inv_RePr;
+  bool factors_ok;  // these are in the estimate's range (dt_factors)
 };
+__device__ __forceinline__ void dt_factors(DtScan& s, double staleT, double inv_Re, double inv_RePr) {
+  s.sqrt_stale = f_sqrt((float)staleT);
+  s.inv_Re = (float)inv_Re;
+  s.inv_RePr = (float)inv_RePr;
+  const float inv = fminf(fabsf(s.inv_Re), fabsf(s.inv_RePr));
+  // (a stale T of zero, as before the first step, leaves no sound term to cover a lost viscous one)
+  s.factors_ok = s.phys || (staleT >= DT_NORMAL ? inv >= DT_NORMAL : staleT == 0.0 && inv >= 1.0e-12f);
+}
 
 // One strip of 32 columns x K rows, by one warp; SCREEN: as above, else every point in FP64.
 // blanked(o): whether the point at offset o is blanked (counted in nblank); exact(i, j, o): the
@@ -109,6 +126,7 @@ __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, u
     const float x = (float)__ldg(s.dxidz + i);
     const float yl = (float)__ldg(s.detadr + j0 + min((int)lane, nrow - 1));
     float up[K];      // upper bound of x
+    float nz[K];      // zero: a part underflowed
     float lo = 0.0f;  // largest lower bound
 #pragma unroll
     for (int k = 0; k < K; ++k) {
@@ -116,8 +134,10 @@ __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, u
       const float Vr = (float)vr[k], Vz = (float)vz[k], T = (float)tt[k];
       const float a = Vz * x, b = Vr * y;
       const float g2 = x * x + y * y;
-      const float snd = s.phys ? f_sqrt(T) * f_sqrt(g2) : s.sqrt_stale * f_sqrt(g2);
+      const float gs = f_sqrt(g2);
+      const float snd = (s.phys ? f_sqrt(T) : s.sqrt_stale) * gs;
       const float mu = f_ex2(0.666f * f_lg2(T));
+      nz[k] = mu * gs;
       const float lam = (0.6f - 2.0f / 3.0f) * mu;
       const float mx = fmaxf(fmaxf(mu, lam) * s.inv_Re, mu * s.inv_RePr);
       const float d = fabsf(x) + fabsf(y);
@@ -143,10 +163,10 @@ __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, u
       if (h > b) atomicMax(sL, h);  // for the strips to come
       else if (h < b) atomicMax(hint, b);
     }
-    const float thr = __uint_as_float(b);
+    const float thr = s.factors_ok ? __uint_as_float(b) : -1.0f / 0.0f;
 #pragma unroll
     for (int k = 0; k < K; ++k)
-      if (up[k] < thr) cand &= ~(1u << k);
+      if (up[k] < thr && nz[k] > 0.0f) cand &= ~(1u << k);
   } else {
 #pragma unroll
     for (int k = 0; k < K; ++k)

@@ -1078,9 +1078,7 @@ __device__ __forceinline__ void dt_body(const DtArgs& a, int blk) {
   sc.dxidz = a.dxidz;
   sc.detadr = a.detadr;
   sc.phys = phys;
-  sc.sqrt_stale = f_sqrt((float)Tst);
-  sc.inv_Re = (float)a.c.inv_Re;
-  sc.inv_RePr = (float)a.c.inv_RePr;
+  dt_factors(sc, Tst, a.c.inv_Re, a.c.inv_RePr);
   unsigned* hint = a.counter + 1;
   const unsigned nstrip = (unsigned)dt_strips(sc.Nz, sc.Nr, SCREEN);
   for (unsigned st = blk * DT_WARPS + (threadIdx.x >> 5); st < nstrip; st += a.nblk * DT_WARPS)

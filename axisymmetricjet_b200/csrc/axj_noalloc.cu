@@ -70,9 +70,7 @@ __global__ void __launch_bounds__(NA_THREADS, 4)
   sc.dxidz = dxidz;
   sc.detadr = detadr;
   sc.phys = phys;
-  sc.sqrt_stale = axj::f_sqrt((float)staleT);
-  sc.inv_Re = (float)c.inv_Re;
-  sc.inv_RePr = (float)c.inv_RePr;
+  axj::dt_factors(sc, staleT, c.inv_Re, c.inv_RePr);
   double v = 1.0e300;
   int blank = 0;
   const unsigned nstrip = (unsigned)axj::dt_strips(Nz, Nr, SCREEN);

@@ -76,3 +76,45 @@ def test_handle_without_a_positive_cfl(oracle_mod, Nz, Nr, CFL):
         mz, mr = ora.metrics()[:2]
         got = _call(c["pv"], np.ascontiguousarray(mz[0]), np.ascontiguousarray(mr[:, 0]), c["params"])
         assert abs(got - want) <= TOL * abs(want)
+
+
+@pytest.mark.parametrize("Nz,Nr", SIZES)
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("T", [-1e-40, -1e-300])
+def test_small_negative_temperature(Nz, Nr, mode, T):
+    """T**0.666 of a negative T is not a number, however small it is."""
+    pv, dxidz, detadr = _flow(Nz, Nr)
+    p = axj.default_params(dt_mode=mode)
+    assert _call(pv, dxidz, detadr, p) > 0.0
+    pv[4, Nr // 2, Nz // 3] = T
+    assert np.isnan(_call(pv, dxidz, detadr, p))
+
+
+@pytest.mark.parametrize("Nz,Nr", SIZES)
+@pytest.mark.parametrize("kind", ["metrics", "temperature", "viscosity", "velocity", "no sound"])
+def test_below_single_precision(Nz, Nr, kind):
+    """Rates whose parts are below FP32's normal range."""
+    pv, dxidz, detadr = _flow(Nz, Nr)
+    p, stale = axj.default_params(dt_mode=1), None
+    if kind == "metrics":  # lengths of 1e19 units
+        dxidz, detadr = np.full(Nz, 5e-20), np.zeros(Nr)
+        pv[3] = 0.5
+        pv[4] = 1.0
+        pv[3, Nr // 2, Nz // 3], pv[4, Nr // 2, Nz // 3] = 0.4, 9.0
+    elif kind == "temperature":
+        pv[1] = pv[3] = 0.0
+        pv[4] *= 1e-40
+    elif kind == "viscosity":
+        pv[1] = pv[3] = 0.0
+        p, stale = axj.default_params(dt_mode=0, Re=1e44), 0.0
+    elif kind == "no sound":  # the stale T before the first step
+        pv[1] = pv[3] = 0.0
+        p, stale = axj.default_params(dt_mode=0), 0.0
+    else:  # an advection rate of order one from a velocity below and a metric far above
+        pv[1] = 0.0
+        pv[3] *= 1e-45
+        p, stale = axj.default_params(dt_mode=0, Re=1e300), 0.0
+        dxidz, detadr = dxidz * 1e36, detadr * 1e-3
+    want = _dts(pv, dxidz, detadr, p, stale).min()
+    got = _call(pv, dxidz, detadr, p, 1.0 if stale is None else stale)
+    assert abs(got - want) <= TOL * want
