@@ -14,10 +14,8 @@
 // underflows (below) are always evaluated in FP64. The largest lower bound seen so far is handed
 // from block to block through a word in global memory (a hint: any value it holds is a valid
 // bound), so that most blocks evaluate no point in FP64 at all.
-// Measured at 4400 x 640 on a B200: the allocation-free kernel 51.4 -> 19.7 us (a call 57.4 ->
-// 22.6 us), the handle's 35.7 -> 23.0 us; what remains is issue (62 % of the active cycles) and
-// the launch's head and tail. Unscreened at 512 x 128 (one strip row per warp, a grid sized to
-// the points): 6.8 -> 5.5 us.
+// Measured at 4400 x 640 on a B200: a call of the allocation-free entry point 55.4 -> 22.3 us, the
+// handle's kernel 27.0 -> 20.1 us.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -26,28 +24,31 @@
 
 namespace axj {
 
-// A warp takes a strip of 32 columns by DT_K rows (1 row where the scan is not screened): the
-// z metric is loaded and converted once per strip, the row's by one lane, and rows shorter
-// than a block waste at most part of a strip.
+// Screened, a warp takes strips of 32 columns by DT_K rows: the z metric is loaded and converted
+// once per strip, the row's by one lane. Otherwise one point per thread, in row order.
 constexpr int DT_K = 4;
 constexpr int DT_WARPS = DT_THREADS / 32;
-// Grids up to this many points are scanned in FP64 throughout, one point per thread: the
-// screen's second pass then costs more than the FP64 work it saves. Measured (full / screened),
-// the handle's kernel: 38,400 points 5.2 / 6.1 us, 180,000 9.5 / 6.3, 400,000 13.2 / 8.1, 1.28 M
-// 34 / 14.6; a call of the allocation-free entry point: 65,536 points 11.6 / 11.6 us, 180,000
-// 12.3 / 10.4, 400,000 16.4 / 10.9, 2.8 M 63.6 / 22.5.
+// A scan in FP64 throughout takes 8.5 us + 19 ps a point (a call of the allocation-free entry
+// point on a B200), a screened one 9.6 us + 4.6 ps for each of its strips' 32-column slots, used
+// or not: the screened one wins above DT_FULL points in full strips, above ever more
+// points the more slots are idle, and in no grid of 10 columns or fewer. Measured (FP64 / screened):
+// 256 x 384 10.1 / 10.3 us, 787 x 203 10.8 / 10.3, 1801 x 333 18.5 / 12.4, 4400 x 640 55 / 22; 33 x 10000
+// 14.0 / 13.1, 12 x 20000 12.5 / 12.8, 12 x 200000 47 / 37, 8 x 500000 78 / 81, 1 x 2097152 42 / 287.
 constexpr long long DT_FULL = 98304;
-__host__ __device__ constexpr bool dt_screened(long long npts) { return npts > DT_FULL; }
-__host__ __device__ constexpr int dt_rows(bool screen) { return screen ? DT_K : 1; }
-// Strips of a grid, and the blocks that take one strip per warp.
-__host__ __device__ inline long long dt_strips(int Nz, int Nr, bool screen) {
-  const int K = dt_rows(screen);
-  return (long long)((Nz + 31) / 32) * ((Nr + K - 1) / K);
+__host__ __device__ inline bool dt_screened(int Nz, int Nr) {
+  const long long n = (long long)Nz * Nr, slots = (long long)((Nz + 31) / 32 * 32) * Nr;
+  return 3 * n > slots + 2 * DT_FULL;
 }
-constexpr long long DT_WAVE = 148 * 4;  // blocks of a screened scan: one resident wave
+// Strips of a screened grid, and a scan's blocks: a strip per warp up to one resident wave, or a
+// point per thread.
+__host__ __device__ inline long long dt_strips(int Nz, int Nr) {
+  return (long long)((Nz + 31) / 32) * ((Nr + DT_K - 1) / DT_K);
+}
+constexpr long long DT_WAVE = 148 * 4;
 __host__ __device__ inline long long dt_blocks(int Nz, int Nr, bool screen) {
-  const long long b = (dt_strips(Nz, Nr, screen) + DT_WARPS - 1) / DT_WARPS;
-  return screen && b > DT_WAVE ? DT_WAVE : b;
+  if (!screen) return ((long long)Nz * Nr + DT_THREADS - 1) / DT_THREADS;
+  const long long b = (dt_strips(Nz, Nr) + DT_WARPS - 1) / DT_WARPS;
+  return b < DT_WAVE ? b : DT_WAVE;
 }
 constexpr float DT_SCREEN = 1.220703125e-4f;   // 2**-13
 constexpr float DT_TINY = 1.0e-30f;            // absolute margin (subnormal products)
@@ -95,14 +96,15 @@ __device__ __forceinline__ void dt_factors(DtScan& s, double staleT, double inv_
   s.factors_ok = s.phys || (staleT >= DT_NORMAL ? inv >= DT_NORMAL : staleT == 0.0 && inv >= 1.0e-12f);
 }
 
-// One strip of 32 columns x K rows, by one warp; SCREEN: as above, else every point in FP64.
-// blanked(o): whether the point at offset o is blanked (counted in nblank); exact(i, j, o): the
-// FP64 evaluation. sL: the largest lower bound the block knows (float bits in shared memory,
-// zeroed by the caller before a barrier; it only grows, any value it holds is a valid bound, and
-// no warp waits for another's); hint: the launch's.
-template <int K, bool SCREEN, class Blanked, class Exact>
+// One strip of 32 columns x DT_K rows of a screened scan, by one warp. blanked(o): whether the
+// point at offset o is blanked (counted in nblank); exact(i, j, o): the FP64 evaluation. sL: the
+// largest lower bound the block knows (float bits in shared memory, zeroed by the caller before
+// a barrier; it only grows, any value it holds is a valid bound, and no warp waits for
+// another's); hint: the launch's.
+template <class Blanked, class Exact>
 __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, unsigned* sL, unsigned* hint,
                                               int& nblank, Blanked blanked, Exact exact) {
+  constexpr int K = DT_K;
   // (a grid that fits the device has far fewer than 2**31 strips)
   const unsigned ncs = (unsigned)(s.Nz + 31) / 32u, lane = threadIdx.x & 31u;
   const unsigned rg = strip / ncs;
@@ -110,74 +112,86 @@ __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, u
   const int iu = (int)((strip - rg * ncs) * 32u + lane), i = min(iu, s.Nz - 1);
   const long long o0 = (long long)j0 * s.P + i;
   unsigned cand = 0;  // rows to evaluate in FP64
-  if constexpr (SCREEN) {
-    // every load of the strip first (none depends on another), then the estimates
-    double vr[K], vz[K], tt[K];
-    bool bl[K];
-    const double* u = s.U + o0;
+  // every load of the strip first (none depends on another), then the estimates
+  double vr[K], vz[K], tt[K];
+  bool bl[K];
+  const double* u = s.U + o0;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const long long o = min(k, nrow - 1) * s.P;  // rows past the grid repeat the last one
-      bl[k] = blanked(o0 + o);
-      vr[k] = __ldg(u + s.plane + o);
-      vz[k] = __ldg(u + 3 * s.plane + o);
-      tt[k] = __ldg(u + 4 * s.plane + o);
-    }
-    const float x = (float)__ldg(s.dxidz + i);
-    const float yl = (float)__ldg(s.detadr + j0 + min((int)lane, nrow - 1));
-    float up[K];      // upper bound of x
-    float nz[K];      // zero: a part underflowed
-    float lo = 0.0f;  // largest lower bound
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const float y = __shfl_sync(0xffffffffu, yl, k);
-      const float Vr = (float)vr[k], Vz = (float)vz[k], T = (float)tt[k];
-      const float a = Vz * x, b = Vr * y;
-      const float g2 = x * x + y * y;
-      const float gs = f_sqrt(g2);
-      const float snd = (s.phys ? f_sqrt(T) : s.sqrt_stale) * gs;
-      const float mu = f_ex2(0.666f * f_lg2(T));
-      nz[k] = mu * gs;
-      const float lam = (0.6f - 2.0f / 3.0f) * mu;
-      const float mx = fmaxf(fmaxf(mu, lam) * s.inv_Re, mu * s.inv_RePr);
-      const float d = fabsf(x) + fabsf(y);
-      const float visc = 2.0f * mx * (d * d);
-      const float est = fabsf(a + b) + snd + visc;
-      const float mar = DT_SCREEN * (fabsf(a) + fabsf(b) + snd + fabsf(visc)) + DT_TINY;
-      up[k] = est + mar;
-      // (a repeated row or column counts once more: the same bound, no point of its own)
-      if (bl[k]) {
-        nblank = 1;
-      } else {
-        lo = fmaxf(lo, est - mar);  // (fmaxf drops a NaN)
-        if (k < nrow && iu < s.Nz) cand |= 1u << k;
-      }
-    }
-    // a lower bound that overflowed says nothing
-    const unsigned lob = lo <= 3.0e38f ? __float_as_uint(lo) : 0u;
-    const unsigned w = __reduce_max_sync(0xffffffffu, lob);
-    const unsigned b = max(*reinterpret_cast<volatile unsigned*>(sL), w);
-    if (lane == 0 && b == w) atomicMax(sL, w);
-    if (threadIdx.x == 0) {
-      const unsigned h = *reinterpret_cast<volatile unsigned*>(hint);
-      if (h > b) atomicMax(sL, h);  // for the strips to come
-      else if (h < b) atomicMax(hint, b);
-    }
-    const float thr = s.factors_ok ? __uint_as_float(b) : -1.0f / 0.0f;
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (up[k] < thr && nz[k] > 0.0f) cand &= ~(1u << k);
-  } else {
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      if (k < nrow && iu < s.Nz) {
-        if (blanked(o0 + k * s.P)) nblank = 1;
-        else cand |= 1u << k;
-      }
+  for (int k = 0; k < K; ++k) {
+    const long long o = min(k, nrow - 1) * s.P;  // rows past the grid repeat the last one
+    bl[k] = blanked(o0 + o);
+    vr[k] = __ldg(u + s.plane + o);
+    vz[k] = __ldg(u + 3 * s.plane + o);
+    tt[k] = __ldg(u + 4 * s.plane + o);
   }
+  const float x = (float)__ldg(s.dxidz + i);
+  const float yl = (float)__ldg(s.detadr + j0 + min((int)lane, nrow - 1));
+  float up[K];      // upper bound of x
+  float nz[K];      // zero: a part underflowed
+  float lo = 0.0f;  // largest lower bound
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const float y = __shfl_sync(0xffffffffu, yl, k);
+    const float Vr = (float)vr[k], Vz = (float)vz[k], T = (float)tt[k];
+    const float a = Vz * x, b = Vr * y;
+    const float g2 = x * x + y * y;
+    const float gs = f_sqrt(g2);
+    const float snd = (s.phys ? f_sqrt(T) : s.sqrt_stale) * gs;
+    const float mu = f_ex2(0.666f * f_lg2(T));
+    nz[k] = mu * gs;
+    const float lam = (0.6f - 2.0f / 3.0f) * mu;
+    const float mx = fmaxf(fmaxf(mu, lam) * s.inv_Re, mu * s.inv_RePr);
+    const float d = fabsf(x) + fabsf(y);
+    const float visc = 2.0f * mx * (d * d);
+    const float est = fabsf(a + b) + snd + visc;
+    const float mar = DT_SCREEN * (fabsf(a) + fabsf(b) + snd + fabsf(visc)) + DT_TINY;
+    up[k] = est + mar;
+    // (a repeated row or column counts once more: the same bound, no point of its own)
+    if (bl[k]) {
+      nblank = 1;
+    } else {
+      lo = fmaxf(lo, est - mar);  // (fmaxf drops a NaN)
+      if (k < nrow && iu < s.Nz) cand |= 1u << k;
+    }
+  }
+  // a lower bound that overflowed says nothing
+  const unsigned lob = lo <= 3.0e38f ? __float_as_uint(lo) : 0u;
+  const unsigned w = __reduce_max_sync(0xffffffffu, lob);
+  const unsigned b = max(*reinterpret_cast<volatile unsigned*>(sL), w);
+  if (lane == 0 && b == w) atomicMax(sL, w);
+  if (threadIdx.x == 0) {
+    const unsigned h = *reinterpret_cast<volatile unsigned*>(hint);
+    if (h > b) atomicMax(sL, h);  // for the strips to come
+    else if (h < b) atomicMax(hint, b);
+  }
+  const float thr = s.factors_ok ? __uint_as_float(b) : -1.0f / 0.0f;
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (up[k] < thr && nz[k] > 0.0f) cand &= ~(1u << k);
 #pragma unroll 1
   for (int k = 0; k < K; ++k)
     if ((cand >> k) & 1u) exact(i, j0 + k, o0 + k * s.P);
+}
+
+// The points of block blk of nblk.
+template <bool SCREEN, class Blanked, class Exact>
+__device__ __forceinline__ void dt_scan(const DtScan& s, unsigned blk, unsigned nblk, unsigned* sL, unsigned* hint,
+                                        int& nblank, Blanked blanked, Exact exact) {
+  if constexpr (SCREEN) {
+    const unsigned n = (unsigned)dt_strips(s.Nz, s.Nr);
+    for (unsigned st = blk * DT_WARPS + (threadIdx.x >> 5); st < n; st += nblk * DT_WARPS)
+      dt_scan_strip(s, st, sL, hint, nblank, blanked, exact);
+  } else {
+    // (a grid that fits the device has fewer than 2**32 points)
+    const unsigned n = (unsigned)s.Nz * (unsigned)s.Nr, step = nblk * DT_THREADS;
+    for (unsigned p = blk * DT_THREADS + threadIdx.x; p < n; p += step) {
+      const int j = (int)(p / (unsigned)s.Nz), i = (int)(p - (unsigned)j * (unsigned)s.Nz);
+      const long long o = (long long)j * s.P + i;
+      if (blanked(o)) nblank = 1;
+      else exact(i, j, o);
+      if (p + step < p) break;
+    }
+  }
 }
 
 }  // namespace axj

@@ -1080,27 +1080,25 @@ __device__ __forceinline__ void dt_body(const DtArgs& a, int blk) {
   sc.phys = phys;
   dt_factors(sc, Tst, a.c.inv_Re, a.c.inv_RePr);
   unsigned* hint = a.counter + 1;
-  const unsigned nstrip = (unsigned)dt_strips(sc.Nz, sc.Nr, SCREEN);
-  for (unsigned st = blk * DT_WARPS + (threadIdx.x >> 5); st < nstrip; st += a.nblk * DT_WARPS)
-    dt_scan_strip<dt_rows(SCREEN), SCREEN>(
-        sc, st, &sL, hint, blank, [&](long long o) { return desc_blank(__ldg(a.desc + o)); },
-        [&](int i, int j, long long o) {
-          const double Vr = __ldg(a.U + 1 * PL + o), Vz = __ldg(a.U + 3 * PL + o), T = __ldg(a.U + 4 * PL + o);
-          const double dxidz = __ldg(a.dxidz + i), detadr = __ldg(a.detadr + j);
-          const double mu = mu_k<double>(T);
-          const double beta = (3.0 / 5.0) * mu;
-          const double lambda = beta - (2.0 / 3.0) * mu;
-          // dt_point's denominator, term for term
-          const double inv =
-              fabs(Vz * dxidz + Vr * detadr) + sqrt(phys ? T : Tst) * sqrt(dxidz * dxidz + detadr * detadr);
-          double mx = (lambda > mu ? lambda : mu) * a.c.inv_Re;
-          const double k = mu * a.c.inv_RePr;
-          if (k > mx) mx = k;
-          const double sabs = fabs(dxidz) + fabs(detadr);
-          const double x = inv + 2.0 * mx * (sabs * sabs);
-          if (!isfinite(x)) bad = 1;  // NaN, or an infinite input (which would give dt = 0)
-          xm = fmax(xm, pos ? x : -(a.c.CFL / x));
-        });
+  dt_scan<SCREEN>(
+      sc, blk, a.nblk, &sL, hint, blank, [&](long long o) { return desc_blank(__ldg(a.desc + o)); },
+      [&](int i, int j, long long o) {
+        const double Vr = __ldg(a.U + 1 * PL + o), Vz = __ldg(a.U + 3 * PL + o), T = __ldg(a.U + 4 * PL + o);
+        const double dxidz = __ldg(a.dxidz + i), detadr = __ldg(a.detadr + j);
+        const double mu = mu_k<double>(T);
+        const double beta = (3.0 / 5.0) * mu;
+        const double lambda = beta - (2.0 / 3.0) * mu;
+        // dt_point's denominator, term for term
+        const double inv =
+            fabs(Vz * dxidz + Vr * detadr) + sqrt(phys ? T : Tst) * sqrt(dxidz * dxidz + detadr * detadr);
+        double mx = (lambda > mu ? lambda : mu) * a.c.inv_Re;
+        const double k = mu * a.c.inv_RePr;
+        if (k > mx) mx = k;
+        const double sabs = fabs(dxidz) + fabs(detadr);
+        const double x = inv + 2.0 * mx * (sabs * sabs);
+        if (!isfinite(x)) bad = 1;  // NaN, or an infinite input (which would give dt = 0)
+        xm = fmax(xm, pos ? x : -(a.c.CFL / x));
+      });
   const bool anyblank = __syncthreads_or(blank);
   xm = warp_max(xm);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1174,10 +1172,9 @@ cudaError_t launch_harmonic_phase(const double* time, const double* dt, double o
   return cudaGetLastError();
 }
 
-bool dt_grid_screened(int Nz, int Nr, const Consts& c) { return dt_screened((long long)Nz * Nr) && c.CFL > 0.0; }
+bool dt_grid_screened(int Nz, int Nr, const Consts& c) { return dt_screened(Nz, Nr) && c.CFL > 0.0; }
 
-// Blocks of the dt kernel: one resident wave of a screened scan, else one strip row per warp, as far
-// as there are places for their minima (the blocks loop).
+// Blocks of the dt kernel, as far as there are places for their minima (the blocks loop).
 int dt_grid_blocks(int Nz, int Nr, const Consts& c) {
   return (int)std::min<long long>(dt_blocks(Nz, Nr, dt_grid_screened(Nz, Nr, c)), DT_MAX_BLOCKS);
 }

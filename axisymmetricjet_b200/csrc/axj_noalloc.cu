@@ -44,13 +44,14 @@ __device__ __forceinline__ double na_warp_min(double v) {
 }
 
 // Per-point dt of ComputeTimeStep (ModInputOutput.f90:395-416), block minimum, and the
-// last block to finish reduces the per-block minima. A block takes one strip per warp
-// of the shared point scan (axj_dt.cuh). The largest rate is the smallest dt only for a positive
+// last block to finish reduces the per-block minima. The points are scanned as the handles'
+// kernel scans them (axj_dt.cuh). The largest rate is the smallest dt only for a positive
 // CFL, and the estimate's viscous part is the rate's only for positive Re and Pr (dt_point takes the
 // largest of the quotients, of which a negative Re makes another one than the estimate's):
-// anything else, NaN among it, turns the screening off.
+// anything else, NaN among it, turns the screening off. (Unscreened, six blocks per SM: at the 62
+// registers the compiler takes for four, 4 x 1000000 points took 103 us, at 42 80 us.)
 template <bool SCREEN>
-__global__ void __launch_bounds__(NA_THREADS, 4)
+__global__ void __launch_bounds__(NA_THREADS, SCREEN ? 4 : 6)
     dt_noalloc_kernel(const double* __restrict__ U, long long P, long long plane, int Nz, int Nr,
                       const double* __restrict__ dxidz, const double* __restrict__ detadr,
                       const double* __restrict__ ibval, double staleT, axj::Consts c, double* scratch,
@@ -73,21 +74,19 @@ __global__ void __launch_bounds__(NA_THREADS, 4)
   axj::dt_factors(sc, staleT, c.inv_Re, c.inv_RePr);
   double v = 1.0e300;
   int blank = 0;
-  const unsigned nstrip = (unsigned)axj::dt_strips(Nz, Nr, SCREEN);
-  for (unsigned st = blockIdx.x * axj::DT_WARPS + (threadIdx.x >> 5); st < nstrip; st += gridDim.x * axj::DT_WARPS)
-    axj::dt_scan_strip<axj::dt_rows(SCREEN), SCREEN>(
-        sc, st, &sL, counter + 1, blank, [&](long long o) { return ibval && __ldg(ibval + o) == 0.0; },
-        [&](int i, int j, long long o) {
-          const double Vr = __ldg(U + 1 * plane + o), Vz = __ldg(U + 3 * plane + o), T = __ldg(U + 4 * plane + o);
-          // mu = T**0.666 (AssignValues) from the table-driven power of the handle-based kernels
-          const double mu = axj::pow0666(T, g_na_pow);
-          const double beta = (3.0 / 5.0) * mu;
-          const double lambda = beta - (2.0 / 3.0) * mu;
-          const double x = axj::dt_point(Vz, Vr, phys ? T : staleT, mu, lambda, mu, __ldg(dxidz + i), __ldg(detadr + j), c);
-          // an infinite input gives dt = 0, a finite-looking minimum: flag it with the NaNs
-          if (!isfinite(Vr) || !isfinite(Vz) || !isfinite(T) || !(x == x)) atomicOr(bad, 1u);
-          v = fmin(v, x);
-        });
+  axj::dt_scan<SCREEN>(
+      sc, blockIdx.x, gridDim.x, &sL, counter + 1, blank, [&](long long o) { return ibval && __ldg(ibval + o) == 0.0; },
+      [&](int i, int j, long long o) {
+        const double Vr = __ldg(U + 1 * plane + o), Vz = __ldg(U + 3 * plane + o), T = __ldg(U + 4 * plane + o);
+        // mu = T**0.666 (AssignValues) from the table-driven power of the handle-based kernels
+        const double mu = axj::pow0666(T, g_na_pow);
+        const double beta = (3.0 / 5.0) * mu;
+        const double lambda = beta - (2.0 / 3.0) * mu;
+        const double x = axj::dt_point(Vz, Vr, phys ? T : staleT, mu, lambda, mu, __ldg(dxidz + i), __ldg(detadr + j), c);
+        // an infinite input gives dt = 0, a finite-looking minimum: flag it with the NaNs
+        if (!isfinite(Vr) || !isfinite(Vz) || !isfinite(T) || !(x == x)) atomicOr(bad, 1u);
+        v = fmin(v, x);
+      });
   if (blank) v = fmin(v, 100.0);
   __shared__ double sred[NA_THREADS / 32];
   __shared__ bool last;
@@ -183,8 +182,7 @@ extern "C" int axj_compute_dt_noalloc(const double* d_pv, int64_t pitch, int64_t
   // before they are read
   cudaError_t e = cudaMemsetAsync(scratch + NA_COUNTER, 0, 2 * sizeof(double), s);
   if (e == cudaSuccess) {
-    const long long n = Nz * Nr;
-    const bool screen = axj::dt_screened(n) && c.CFL > 0.0 && c.Re > 0.0 && c.Pr > 0.0;
+    const bool screen = axj::dt_screened((int)Nz, (int)Nr) && c.CFL > 0.0 && c.Re > 0.0 && c.Pr > 0.0;
     const long long need = axj::dt_blocks((int)Nz, (int)Nr, screen);
     const int blocks = (int)(need < NA_MAX_BLOCKS ? need : NA_MAX_BLOCKS);
     auto kernel = screen ? dt_noalloc_kernel<true> : dt_noalloc_kernel<false>;

@@ -118,3 +118,13 @@ def test_below_single_precision(Nz, Nr, kind):
     want = _dts(pv, dxidz, detadr, p, stale).min()
     got = _call(pv, dxidz, detadr, p, 1.0 if stale is None else stale)
     assert abs(got - want) <= TOL * want
+
+
+@pytest.mark.parametrize("Nz,Nr", [(1, 98305), (4, 100000), (10, 60000), (11, 196608), (11, 196609), (12, 49152),
+                                   (12, 49153), (16, 12289), (31, 3300), (33, 4500), (33, 7000), (65, 1513)])
+def test_narrow_grids(Nz, Nr):
+    """Grids either side of the rule that screens rows of few columns only above more points."""
+    pv, dxidz, detadr = _flow(Nz, Nr, Nz + Nr)
+    p = axj.default_params(dt_mode=1)
+    want = _dts(pv, dxidz, detadr, p).min()
+    assert abs(_call(pv, dxidz, detadr, p) - want) <= TOL * want
