@@ -695,7 +695,7 @@ cudaError_t launch_sample(const Dataset& d, MlpNorm norm, unsigned long long see
 // Here a persistent CTA per SM takes tiles of TB = 128 points: the gathered inputs, both
 // hidden layers and the weights (in both orientations) stay in its shared memory, the
 // pre-activations of a thread's 8 x 4 block in its registers, and the weight gradients
-// accumulate in registers over all of the CTA's tiles; they leave once, as rows of `part`
+// accumulate in registers over up to TFLUSH of the CTA's tiles and then go to rows of `part`
 // (two per CTA), which the update kernel sums in a fixed order: a step is deterministic.
 // Thread blocks of 8 x 4 outputs read 3 float4 of shared memory per 32 FMA (forward and input
 // gradients: points ty + 16 r, columns 4 tx..), of 8 x 7 and 8 x 4 in the weight gradients
@@ -707,6 +707,10 @@ cudaError_t launch_sample(const Dataset& d, MlpNorm norm, unsigned long long see
 // ---------------------------------------------------------------------------
 constexpr int TB = 128;         // points per tile
 constexpr int TT = 256;         // threads
+// Tiles whose weight gradients are summed in registers before they are added to the rows of part:
+// no sum runs over more than 8 * 64 points one by one. Over all of a CTA's tiles the rounding of
+// 2**21 points grew to 7e-5 of an entry (sums of 1024: 2e-5).
+constexpr int TFLUSH = 8;
 constexpr int TXP = MLP_K1 + 4;  // row pitch of the input tile (float4 rows, banks of adjacent rows apart)
 constexpr int THP = MLP_HID + 4;
 struct TrainSmem {
@@ -791,6 +795,9 @@ __global__ void __launch_bounds__(TT, 1)
   gb3[0] = gb3[1] = 0.0f;
   const float invB = 1.0f / (float)B;
   const int ntile = (B + TB - 1) / TB;
+  float* row = part + (long long)(2 * blockIdx.x + half) * MLP_NPARAM;
+  int held = 0;  // tiles summed in the registers
+  bool first = true;
   for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
     const int b0 = tile * TB;
     __syncthreads();  // the previous tile's reads of X, D and T are done
@@ -961,17 +968,33 @@ __global__ void __launch_bounds__(TT, 1)
         for (int c = 0; c < 8; ++c) g1[c][t] = fmaf(a[c], x, g1[c][t]);
       }
     }
+    // ---- the weight gradients of these tiles to the half's row of part (eleven loads in flight)
+    if (++held == TFLUSH || tile + gridDim.x >= ntile) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        float* w1 = row + MLP_OFF_W1 + (8 * ng + c) * MLP_K1 + kg;
+        float* w2 = row + MLP_OFF_W2 + (8 * ng + c) * MLP_HID + 4 * kg;
+        float s1[7], s2[4];
+#pragma unroll
+        for (int t = 0; t < 7; ++t) s1[t] = first ? 0.0f : w1[16 * t];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s2[q] = first ? 0.0f : w2[q];
+#pragma unroll
+        for (int t = 0; t < 7; ++t) {
+          w1[16 * t] = s1[t] + g1[c][t];
+          g1[c][t] = 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          w2[q] = s2[q] + g2[c][q];
+          g2[c][q] = 0.0f;
+        }
+      }
+      first = false;
+      held = 0;
+    }
   }
-  // ---- the CTA's sums: its two halves' weight gradients as two rows of part, everything
-  // else reduced over ty into the first
-  float* row = part + (long long)(2 * blockIdx.x + half) * MLP_NPARAM;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-#pragma unroll
-    for (int t = 0; t < 7; ++t) row[MLP_OFF_W1 + (8 * ng + c) * MLP_K1 + kg + 16 * t] = g1[c][t];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) row[MLP_OFF_W2 + (8 * ng + c) * MLP_HID + 4 * kg + q] = g2[c][q];
-  }
+  // ---- the CTA's other sums, reduced over ty into its first row
   __syncthreads();  // every thread is done with the tile buffers
   float* red = &s.X[0][0];  // [16][4 x 64 + 4]
   constexpr int RP = 4 * MLP_HID + 4;
