@@ -599,8 +599,7 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       dr.dVtdz = dst6<R, C, 1>(q, pVt, 1) * xz;
       dr.dVzdz = sDz[RR * TZ + dzi];
       dr.dTdz = dst6<R, C, 1>(q, pT, 1) * xz;
-      // (a blanked point's products may overflow where its values do not: zero times infinity)
-      dr.dpdz = C || zr < 9 ? dst6_p<R, C>(q, pR, pT, 1) * xz : R(0);
+      dr.dpdz = dst6_p<R, C>(q, pR, pT, 1) * xz;
       dr.d2Vrdz2 = dst6<R, C, 2>(q, pVr, 1) * (xz * xz) + dr.dVrdz * xzz;
       dr.d2Vtdz2 = dst6<R, C, 2>(q, pVt, 1) * (xz * xz) + dr.dVtdz * xzz;
       dr.d2Vzdz2 = dst6<R, C, 2>(q, pVz, 1) * (xz * xz) + dr.dVzdz * xzz;
@@ -617,7 +616,7 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       dr.dVtdr = dst6<R, C, 1>(q, pVt, RZ) * er;
       dr.dVzdr = dst6<R, C, 1>(q, pVz, RZ) * er;
       dr.dTdr = dst6<R, C, 1>(q, pT, RZ) * er;
-      dr.dpdr = C || rw < 9 ? dst6_p<R, C>(q, pR, pT, RZ) * er : R(0);
+      dr.dpdr = dst6_p<R, C>(q, pR, pT, RZ) * er;
       dr.d2Vrdr2 = dst6<R, C, 2>(q, pVr, RZ) * (er * er) + dr.dVrdr * err;
       dr.d2Vtdr2 = dst6<R, C, 2>(q, pVt, RZ) * (er * er) + dr.dVtdr * err;
       dr.d2Vzdr2 = dst6<R, C, 2>(q, pVz, RZ) * (er * er) + dr.dVzdr * err;
@@ -632,6 +631,8 @@ __device__ __forceinline__ bool stage_compute(const StageArgs& a, int i0, int j0
       else along_z(std::false_type{});
       if (r4) along_r(std::true_type{});
       else along_r(std::false_type{});
+      // (a blanked point's products may overflow where its values do not: zero times infinity)
+      if (blank) dr.dpdz = dr.dpdr = R(0);
     } else {
       along_z(std::true_type{});
       along_r(std::true_type{});
