@@ -33,28 +33,30 @@ struct DevBuf {
 }  // namespace
 
 // Page-locked places of 64 bytes for the handles' step scalars: a page-locked allocation takes
-// about 2 ms, half of a small handle's creation, so handles share pages of 64 places. A page is
-// allocated when none has a free place and given back when its last place is.
+// about 2 ms, half of a small handle's creation, so the handles of a device share pages of 64
+// places. A page is allocated when none has a free place and given back when its last place is. It
+// belongs to its device's context: a program that resets one device takes no other's pages.
 namespace {
 struct PinPool {
   static constexpr int kPlaces = 64, kDoubles = 8;
   struct Page {
     double* base;
     uint64_t used;
+    int device;
   };
   std::mutex lock;
   std::vector<Page> pages;
-  double* get() {
+  double* get(int device) {  // the current device
     std::lock_guard<std::mutex> g(lock);
     for (Page& p : pages)
-      if (~p.used) {
+      if (p.device == device && ~p.used) {
         const int k = __builtin_ctzll(~p.used);
         p.used |= 1ull << k;
         return p.base + k * kDoubles;
       }
     void* m = nullptr;
     if (cudaHostAlloc(&m, kPlaces * kDoubles * sizeof(double), cudaHostAllocPortable) != cudaSuccess) return nullptr;
-    pages.push_back(Page{static_cast<double*>(m), 1ull});
+    pages.push_back(Page{static_cast<double*>(m), 1ull, device});
     return pages.back().base;
   }
   void put(double* q) {
@@ -71,7 +73,8 @@ struct PinPool {
     }
   }
 };
-PinPool g_pins;
+// (never destroyed: a handle may be destroyed by a static destructor that runs after this library's)
+PinPool& g_pins = *new PinPool;
 }  // namespace
 
 struct axj_handle {
@@ -1597,7 +1600,7 @@ int axj_create(const axj_params* prm, int64_t Nz, int64_t Nr, const double* zvec
     h->staleT = h->dt + 2;
     h->flags = reinterpret_cast<int*>(h->dt + 3);
   }
-  if (rc == AXJ_OK && !(h->pin = g_pins.get())) rc = fail(h, AXJ_ERR_NOMEM, "page-locked memory for the step scalars");
+  if (rc == AXJ_OK && !(h->pin = g_pins.get(h->device))) rc = fail(h, AXJ_ERR_NOMEM, "page-locked memory for the step scalars");
   h->harm = dalloc<double>(h, 5, &rc);
 
   h->counter = dalloc<unsigned int>(h, 2, &rc);
