@@ -53,12 +53,12 @@ __host__ __device__ inline long long dt_blocks(int Nz, int Nr, bool screen) {
 constexpr float DT_SCREEN = 1.220703125e-4f;   // 2**-13
 constexpr float DT_TINY = 1.0e-30f;            // absolute margin (subnormal products)
 // Underflow: the approximate units flush subnormals, so a T, or a sum of squared metrics, below FP32's
-// normal range loses its part of the estimate, and a T that is negative but small is no NaN. Either
-// makes mu * sqrt(g2) zero, and the point is then evaluated in FP64 whatever its estimate (which,
-// being too small, is still a valid lower bound). With both normal, what else underflows is below
-// the margin, for velocities up to 1e15 or metrics that are zero or normal in FP32; the stale T and
-// the viscous factors are tested once per launch (dt_factors). Overflow needs no test: an
-// infinite estimate is evaluated too.
+// normal range loses its part of the estimate, and a T that is negative but small is no NaN. The
+// points of a lane whose z metric's square or least T is below that range are therefore evaluated
+// in FP64 whatever their estimates (which, being too small, are still valid lower bounds).
+// Otherwise what underflows is below the margin, for velocities up to 1e15 or metrics that are
+// zero or normal in FP32; the stale T and the viscous factors are tested once per launch
+// (dt_factors). Overflow needs no test: an infinite estimate is evaluated too.
 constexpr float DT_NORMAL = 1.17549435e-38f;
 
 __device__ __forceinline__ float f_sqrt(float x) {
@@ -127,8 +127,8 @@ __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, u
   const float x = (float)__ldg(s.dxidz + i);
   const float yl = (float)__ldg(s.detadr + j0 + min((int)lane, nrow - 1));
   float up[K];      // upper bound of x
-  float nz[K];      // zero: a part underflowed
   float lo = 0.0f;  // largest lower bound
+  float tl = DT_NORMAL;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const float y = __shfl_sync(0xffffffffu, yl, k);
@@ -138,7 +138,7 @@ __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, u
     const float gs = f_sqrt(g2);
     const float snd = (s.phys ? f_sqrt(T) : s.sqrt_stale) * gs;
     const float mu = f_ex2(0.666f * f_lg2(T));
-    nz[k] = mu * gs;
+    tl = fminf(tl, T);  // (a NaN makes its own estimate one)
     const float lam = (0.6f - 2.0f / 3.0f) * mu;
     const float mx = fmaxf(fmaxf(mu, lam) * s.inv_Re, mu * s.inv_RePr);
     const float d = fabsf(x) + fabsf(y);
@@ -164,10 +164,11 @@ __device__ __forceinline__ void dt_scan_strip(const DtScan& s, unsigned strip, u
     if (h > b) atomicMax(sL, h);  // for the strips to come
     else if (h < b) atomicMax(hint, b);
   }
-  const float thr = s.factors_ok ? __uint_as_float(b) : -1.0f / 0.0f;
+  const bool ok = s.factors_ok && x * x >= DT_NORMAL && tl >= DT_NORMAL;
+  const float thr = ok ? __uint_as_float(b) : -1.0f / 0.0f;
 #pragma unroll
   for (int k = 0; k < K; ++k)
-    if (up[k] < thr && nz[k] > 0.0f) cand &= ~(1u << k);
+    if (up[k] < thr) cand &= ~(1u << k);
 #pragma unroll 1
   for (int k = 0; k < K; ++k)
     if ((cand >> k) & 1u) exact(i, j0 + k, o0 + k * s.P);
