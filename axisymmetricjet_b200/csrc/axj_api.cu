@@ -587,9 +587,9 @@ std::vector<int2> zr_row_blocks(const std::vector<unsigned char>& rcode, int Nz,
 // run the recurrence alone); two CTAs of an SM take 1.03, three 1.2 times one's time, and more
 // than three run in turns. So small grids take the shortest segments that fill the SMs once and
 // large ones the longest that still leave three CTAs for each SM. Measured on a B200, the picked
-// length first: 787 x 203 16: 15.1 us (32: 17.7, 64: 25.1); 1024 x 256 32: 14.6 (16: 18.9, 48: 17.7);
-// 1801 x 333 48: 21.4 (32: 27.0, 64: 21.2); 2401 x 500 80: 29.6 (64: 37.4, 96: 31.2); 4400 x 640 176:
-// 55.8 (96: 64.7, 272: 68.1).
+// length first: 787 x 203 16: 16.8 us (32: 19.5, 64: 27.5); 1024 x 256 32: 16.1 (16: 20.1, 48: 17.5);
+// 1801 x 333 48: 21.6 (32: 30.2, 64: 23.3); 2401 x 500 80: 30.6 (64: 39.6, 96: 32.7); 4400 x 640 176:
+// 56.9 (96: 68.7, 272: 69.4).
 int zr_pick_segment(const std::vector<std::pair<int, int>>& work, int nsm) {
   int kmax = 1;
   for (const auto& w : work) kmax = std::max(kmax, (w.first + ZRK_BZ - 1) / ZRK_BZ);

@@ -3,7 +3,7 @@
 //
 // dt is the minimum of CFL / x over the points, x the point's inviscid plus viscous rate. In
 // FP64 x costs about fifty instructions per point (two square roots, T**0.666 with its table
-// loads), which bound the kernels at 36-52 us for 2.8 M points when the 24 B/point they read
+// loads), which bound the kernels at 35-48 us for 2.8 M points when the 24 B/point they read
 // take 10 us; but only the points near the largest x need it. A block therefore first forms an
 // FP32 estimate of x for its points with the approximate square root, log2 and exp2 units
 // (relative error of the parts well below 1e-5), takes the largest estimate, and evaluates
@@ -14,8 +14,8 @@
 // underflows (below) are always evaluated in FP64. The largest lower bound seen so far is handed
 // from block to block through a word in global memory (a hint: any value it holds is a valid
 // bound), so that most blocks evaluate no point in FP64 at all.
-// Measured at 4400 x 640 on a B200: a call of the allocation-free entry point 55.4 -> 22.3 us, the
-// handle's kernel 27.0 -> 20.1 us.
+// Measured at 4400 x 640 on a B200: a call of the allocation-free entry point 55.4 -> 22.7 us, the
+// handle's kernel 27.0 -> 20.1 us (within a step, with the state out of the caches, 35.4 -> 21.2).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -44,7 +44,7 @@ __host__ __device__ inline bool dt_screened(int Nz, int Nr) {
 __host__ __device__ inline long long dt_strips(int Nz, int Nr) {
   return (long long)((Nz + 31) / 32) * ((Nr + DT_K - 1) / DT_K);
 }
-constexpr long long DT_WAVE = 148 * 4;
+constexpr long long DT_WAVE = 148 * 4;  // (a launch shape only: the blocks loop, on any number of SMs)
 __host__ __device__ inline long long dt_blocks(int Nz, int Nr, bool screen) {
   if (!screen) return ((long long)Nz * Nr + DT_THREADS - 1) / DT_THREADS;
   const long long b = (dt_strips(Nz, Nr) + DT_WARPS - 1) / DT_WARPS;

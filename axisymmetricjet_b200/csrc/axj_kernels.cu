@@ -972,7 +972,7 @@ static cudaError_t join(const SideStream& side, cudaStream_t s) {
   return cudaStreamWaitEvent(s, side.join, 0);
 }
 
-constexpr int STAGE_WIDE_TILES = 148;  // one general tile per SM
+constexpr int STAGE_WIDE_TILES = 148;  // one general tile per SM (the faster form; both take any number)
 
 template <typename SIN, typename R>
 static cudaError_t launch_stage_pair(const StageArgs& a, int ntiles_int, const int2* tiles_int, const StageMaps& mint,
@@ -2211,10 +2211,10 @@ __global__ void tgfilter_z_rows_kernel_batch(const SensorArgs* __restrict__ argv
 // right of block k-1 that the filter rows reach, and once both are in registers the
 // slot of block k-1 takes block k+1, which lands while block k-1 is filtered.
 // Measured on a B200 (FP64; before: 30 rows per CTA, a point per thread and round, the power's
-// branch between a thread's points, segments of at least 64 positions with 64 of warm-up):
-// 4400 x 640 64 -> 57 us, 1801 x 333 25.4 -> 21.2, 787 x 203 with a blanked lip 38 -> 15.4,
-// 96 x 64 15.2 -> 10. The FP64 pipe is the bound (336 instructions per thread and own block); it
-// is busy about half the time between the phases' barriers.
+// branch between a thread's points, segments of at least 64 positions):
+// 4400 x 640 64 -> 57 us, 1801 x 333 25.4 -> 21.6, 787 x 203 with a blanked lip 38 -> 16.8,
+// 96 x 64 15.2 -> 11.8. Latency bounds it: the recurrence and the points (336 FP64 instructions per
+// thread and own block) alternate between barriers, the FP64 pipe is active 29 % of the time.
 // ---------------------------------------------------------------------------
 constexpr int ZRK_LANES = 3 * ZRK_NR;  // 150 recurrences per CTA
 constexpr int ZRK_QROW = ZRK_BZ * 8;   // bytes of one row of a Q block (128)

@@ -183,8 +183,8 @@ constexpr int ZRK_RBC = 40, ZRK_HRC = 5;      // compact
 constexpr int ZRK_RBW = 30, ZRK_HRW = 10;     // wide
 // Warm-up positions of a segment (4 blocks). What the recurrence forgets before a segment starts is
 // 0.47**64 = 1e-21 of the largest value left of it: below rounding behind fronts of up to five
-// decades. With 48 positions (5e-17 before rounding) values behind a front 1e6 high were off by
-// 2e-11, and the kernel was no faster (787 x 203 15.4 us, 4400 x 640 57; with 64: 15.1 and 56).
+// decades. With 48 positions (2e-16) values behind a front 1e6 high were off by 2e-11; the fourth
+// block costs 1 to 2 us a launch (787 x 203 15.1 -> 16.9 us, 4400 x 640 55.4 -> 57.0).
 constexpr int ZRK_WARM = 64;
 struct ZrArgs {
   Grid g;

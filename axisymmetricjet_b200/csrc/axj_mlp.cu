@@ -700,9 +700,9 @@ cudaError_t launch_sample(const Dataset& d, MlpNorm norm, unsigned long long see
 // Thread blocks of 8 x 4 outputs read 3 float4 of shared memory per 32 FMA (forward and input
 // gradients: points ty + 16 r, columns 4 tx..), of 8 x 7 and 8 x 4 in the weight gradients
 // (half the tile's points per 128 threads), so the FP32 pipe, not shared memory, is the bound.
-// Measured on a B200, a step of 65,536 points: 980 us in 20 launches -> 146 us + 7 us (update);
-// a 20-step training call 25.5 -> 4.6 ms. The FP32 multiply-adds alone take 54 us at the pipe's
-// rate (of which 4 rounds of tiles for 3.5 per SM cost 15 %); the rest is one CTA's barriers,
+// Measured on a B200, a step of 65,536 points: 980 us in 20 launches -> 143 us + 7 us (update);
+// a 20-step training call 25.1 -> 4.1 ms. The FP32 multiply-adds alone take 45 us at the pipe's
+// rate, 52 with four rounds of tiles for 3.46 per SM; the rest is one CTA's barriers,
 // the gather of a tile's windows and the activations.
 // ---------------------------------------------------------------------------
 constexpr int TB = 128;         // points per tile
